@@ -144,7 +144,10 @@ int pf_set_stream(pf_ctx* ctx, void* stream);
 #define PF_OPT_FUSED 1     /* 1 (default): pf_step uses the fused kernels;
                               0: it calls the per-subroutine kernels        */
 #define PF_OPT_TILE_Y 2    /* fused tile height: 4, 8 (default) or 16       */
-#define PF_OPT_ZCHUNK 3    /* z planes per fused CTA (0 = whole column)     */
+#define PF_OPT_ZCHUNK 3    /* z planes per fused CTA (0 = whole column); until
+                              it is set (default 64) the TMA passes take the
+                              chunk that fills the GPU with the domain's
+                              tiles.  Same results.                         */
 #define PF_OPT_KTIMING 4   /* 1: time every fused launch with CUDA events   */
 #define PF_OPT_PAIRED 5    /* two cells per thread on 32 x 8 fused tiles
                               (same results): 1 (default) in FP32, where it

@@ -71,6 +71,9 @@ struct pf_ctx {
     cudaStream_t own_stream;
     cudaStream_t stream;
     int fused, tile_y, zchunk, ktiming, paired;
+    int zchunk_set;          // PF_OPT_ZCHUNK was set; until then the march passes' chunk is fill_zchunk's
+    int zfill[3];            // ... cached by the CTAs an SM holds (index: kMarchOcc)
+    int n_sm;
     int kernel;              // PF_OPT_KERNEL: 1 TMA-staged march passes, 0 the cp.async passes
     int nslot;               // PF_OPT_NSLOT: window mode of the march passes (0: 3)
     CUtensorMap tmap[2];     // tensor maps of the two phase-field buffers (32 x 8 march tiles)
@@ -102,6 +105,10 @@ static int cuda_check(pf_ctx* c, cudaError_t e, const char* what)
     } while (0)
 
 static inline bool is64(const pf_ctx* c) { return c->prec == PF_FP64; }
+
+// CTAs of the march passes an SM holds, for the chunk rule: FP64 with the
+// smooth noise 2, otherwise FP64 and one FP32 cell a thread 3, FP32 pairs 6
+static const int kMarchOcc[3] = {2, 3, 6};
 
 extern "C" {
 
@@ -153,6 +160,13 @@ int pf_create(const pf_grid* g, const pf_params* p, int precision, pf_ctx** out)
     ctx->ktiming = 0;
     ctx->paired = 1;
     cudaGetDevice(&ctx->device);
+    ctx->zchunk_set = 0;
+    ctx->n_sm = 0;
+    cudaDeviceGetAttribute(&ctx->n_sm, cudaDevAttrMultiProcessorCount, ctx->device);
+    if (ctx->n_sm < 1) ctx->n_sm = 1;
+    for (int q = 0; q < 3; ++q)
+        ctx->zfill[q] = fill_zchunk((long long)((g->nx + 31) / 32) * ((g->ny + 7) / 8), g->nz, ctx->n_sm, kMarchOcc[q],
+                                    3.0, 0.14);
     // one allocation: 7 fields + diagnostics partials
     ctx->field_bytes = round_up((size_t)px * g->ny * g->nz * ctx->es + 64, 256);
     ctx->nblk = 592;
@@ -278,6 +292,7 @@ int pf_set_option(pf_ctx* ctx, int opt, int value)
     case PF_OPT_ZCHUNK:
         if (value < 0) return ctx_err(ctx, PF_E_ARG, "zchunk must be >= 0");
         ctx->zchunk = value;
+        ctx->zchunk_set = 1;
         return PF_OK;
     case PF_OPT_KTIMING: ctx->ktiming = value ? 1 : 0; return PF_OK;
     case PF_OPT_PAIRED:
@@ -650,15 +665,17 @@ static int one_step(pf_ctx* ctx)
         // otherwise (default: FP32 only) or the deck draws the smooth noise
         const int lanes = ((ctx->paired == 2 || (ctx->paired == 1 && !is64(ctx))) && p.ruido_tipo != 2) ? 2 : 1;
         const int nslot = ctx->nslot ? ctx->nslot : 3;
+        const int occ_q = (is64(ctx) && p.ruido_tipo == 2) ? 0 : (lanes == 2 && !is64(ctx)) ? 2 : 1;
+        const int zchunk = ctx->zchunk_set ? ctx->zchunk : ctx->zfill[occ_q];
         auto tm_of = [ctx](const void* buf) -> const CUtensorMap& {
             return ctx->tmap[buf == ctx->tmap_buf[0] ? 0 : 1];
         };
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         f.phi_mid = B;
         if (ctx->ktiming) { e0 = new_event(); e1 = new_event(); cudaEventRecord(e0, ctx->stream); }
-        CK(is64(ctx) ? launch_march_first<double>(tm_of(A), ctx->dd, s, f, nsw == 1, lanes, nslot, ctx->zchunk,
+        CK(is64(ctx) ? launch_march_first<double>(tm_of(A), ctx->dd, s, f, nsw == 1, lanes, nslot, zchunk,
                                                   ctx->d_status, ctx->stream)
-                     : launch_march_first<float>(tm_of(A), ctx->dd, s, f, nsw == 1, lanes, nslot, ctx->zchunk,
+                     : launch_march_first<float>(tm_of(A), ctx->dd, s, f, nsw == 1, lanes, nslot, zchunk,
                                                  ctx->d_status, ctx->stream),
            nsw == 1 ? "march step (single sweep)" : "march heat + sweep 1");
         if (ctx->ktiming) { cudaEventRecord(e1, ctx->stream); ctx->ev_first.push_back({e0, e1}); }
@@ -679,9 +696,9 @@ static int one_step(pf_ctx* ctx)
             f2.phi_mid = cur;
             f2.phi_new = oth;
             if (ctx->ktiming) { e0 = new_event(); e1 = new_event(); cudaEventRecord(e0, ctx->stream); }
-            CK(is64(ctx) ? launch_march_last<double>(tm_of(cur), ctx->dd, s, f2, lanes, nslot, ctx->zchunk,
+            CK(is64(ctx) ? launch_march_last<double>(tm_of(cur), ctx->dd, s, f2, lanes, nslot, zchunk,
                                                      ctx->d_status, ctx->stream)
-                         : launch_march_last<float>(tm_of(cur), ctx->dd, s, f2, lanes, nslot, ctx->zchunk,
+                         : launch_march_last<float>(tm_of(cur), ctx->dd, s, f2, lanes, nslot, zchunk,
                                                     ctx->d_status, ctx->stream),
                "march last sweep + solute");
             if (ctx->ktiming) { cudaEventRecord(e1, ctx->stream); ctx->ev_last.push_back({e0, e1}); }

@@ -72,6 +72,46 @@ inline int validate(const pf_grid* g, const pf_params* p, int precision, std::st
     return PF_OK;
 }
 
+// Planes per z-chunk of a z-marching launch over `tiles` column tiles of a grid
+// of nz planes.  A CTA computes its chunk plane after plane, one dependent
+// chain per plane, so a small domain cut into few long chunks leaves most SMs
+// idle and the rest waiting on latency, while many short chunks pay each
+// chunk's prologue (the planes staged and the nodes computed before its first
+// cell, `pro` planes' worth).  Measured on B200 (148 SMs, FP64 passes): one
+// resident CTA takes 2.06 us a plane, three take 2.6 us each, so a plane's
+// time is modelled as 1 + grow (k - 1) with k CTAs resident an SM; beyond
+// `occ` of them the chunks run in waves, whose last one is partly filled.  The
+// chunk count with the least modelled time wins; chunks are of equal length
+// (the last may be shorter) and no longer than kZChunkMax planes, above which
+// nothing is gained.  Against fixed 64-plane chunks: 36x32x48 FP64
+// 217 -> 22 us a step, 64x64x128 FP64 291 -> 58 us, 150x111x190 FP32
+// 343 -> 160 us, 256x256x512 FP32 1.22 -> 1.15 ms, 340x340x700 FP64 unchanged.
+constexpr int kZChunkMax = 128;
+inline int fill_zchunk(long long tiles, int nz, int n_sm, int occ, double pro, double grow)
+{
+    int best_zc = nz < kZChunkMax ? nz : kZChunkMax;
+    double best = 1e300;
+    for (int n = (nz + kZChunkMax - 1) / kZChunkMax, last = 0; n <= nz; ++n) {
+        const int zc = (nz + n - 1) / n;
+        if (zc == last) continue;
+        last = zc;
+        const double per_sm = (double)(tiles * ((nz + zc - 1) / zc)) / (double)n_sm;
+        double t;
+        if (per_sm <= occ) {
+            t = 1.0 + grow * (std::ceil(per_sm) - 1.0);
+        } else {
+            const double w = per_sm / occ;
+            t = (1.0 + grow * (occ - 1)) * (w < 3.0 ? 0.5 * (w + std::ceil(w)) : w + 0.15);
+        }
+        t *= zc + pro;
+        if (t < best) {
+            best = t;
+            best_zc = zc;
+        }
+    }
+    return best_zc;
+}
+
 inline size_t round_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 inline int pitch_of(int nx) { return (int)round_up((size_t)nx, 32); }
 
