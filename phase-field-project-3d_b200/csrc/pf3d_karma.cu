@@ -9,6 +9,7 @@
 #include "../../include/pf3d.h"
 #include "pf3d_hostdesc.h"
 #include "pf3d_karma.cuh"
+#include "pf3d_tmap.h"
 
 using namespace pf3d;
 
@@ -80,8 +81,10 @@ struct pf_karma {
     void* phi[2];
     void* U[2];
     void* dphi;
+    CUtensorMap tm_phi[2], tm_u[2], tm_dphi;   // plane loads of the passes
     int* d_tip;
-    int* h_tip;   // pinned
+    int* d_status;   // kernel status word: 0, or the code a kernel left there
+    int* h_tip;   // pinned: the two tips, the status word
     int cur;      // which phi/U buffer holds the state
     int it;       // steps done
     int zchunk;   // planes per CTA (fill_zchunk)
@@ -153,8 +156,23 @@ int pf_karma_create(const pf_karma_params* p, int precision, pf_karma** out)
     k->U[1] = b + 3 * k->field_bytes;
     k->dphi = b + 4 * k->field_bytes;
     k->d_tip = (int*)(b + 5 * k->field_bytes);
+    k->d_status = k->d_tip + 8;
+    int tm_rc = 0;
+    auto map_of = [&](CUtensorMap* tm, const void* base) {
+        tm_rc |= encode_field_map(tm, base, (int)k->es, p->nx, p->ny, p->nz, px, karma_box_x((int)k->es), kTY + 2);
+    };
+    for (int q = 0; q < 2; ++q) {
+        map_of(&k->tm_phi[q], k->phi[q]);
+        map_of(&k->tm_u[q], k->U[q]);
+    }
+    map_of(&k->tm_dphi, k->dphi);
+    if (tm_rc != 0) {
+        cudaFree(k->base);
+        delete k;
+        return kerr(PF_E_CUDA, "tensor map encoding failed");
+    }
     if ((e = cudaMemset(k->base, 0, 5 * k->field_bytes + 256)) != cudaSuccess ||
-        (e = cudaMallocHost(&k->h_tip, 2 * sizeof(int))) != cudaSuccess ||
+        (e = cudaMallocHost(&k->h_tip, 3 * sizeof(int))) != cudaSuccess ||
         (e = cudaStreamCreateWithFlags(&k->own_stream, cudaStreamNonBlocking)) != cudaSuccess) {
         cudaFree(k->base);
         delete k;
@@ -195,6 +213,18 @@ int pf_karma_set_it(pf_karma* k, int it)
     if (!k || it < 0) return kerr(PF_E_ARG, "bad argument");
     k->it = it;
     return PF_OK;
+}
+
+// waits for the stream; the kernel status word comes with the wait:
+// PF_E_KERNEL when a kernel reported a failure (cleared once reported)
+static int karma_wait(pf_karma* k, const char* what)
+{
+    cudaError_t e = cudaMemcpyAsync(k->h_tip + 2, k->d_status, sizeof(int), cudaMemcpyDeviceToHost, k->stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(k->stream);
+    const int code = e == cudaSuccess ? k->h_tip[2] : 0;
+    if (code != 0) e = cudaMemsetAsync(k->d_status, 0, sizeof(int), k->stream);
+    if (e != cudaSuccess) return kerr(PF_E_CUDA, std::string(what) + ": " + cudaGetErrorString(e));
+    return code == 0 ? PF_OK : kerr(PF_E_KERNEL, std::string(what) + ": a kernel reported failure code " + std::to_string(code));
 }
 
 static void* karma_field(pf_karma* k, int field)
@@ -239,8 +269,9 @@ int pf_karma_download(pf_karma* k, int field, double* host)
     }
     cudaError_t e = cudaMemcpy2DAsync(dst, (size_t)p.nx * k->es, karma_field(k, field), (size_t)k->d.px * k->es,
                                       (size_t)p.nx * k->es, (size_t)p.ny * p.nz, cudaMemcpyDeviceToHost, k->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(k->stream);
     if (e != cudaSuccess) return kerr(PF_E_CUDA, std::string("download: ") + cudaGetErrorString(e));
+    const int rc = karma_wait(k, "download");
+    if (rc != PF_OK) return rc;
     if (k->prec == PF_FP32)
         for (size_t q = 0; q < n; ++q) host[q] = (double)tmp[q];
     return PF_OK;
@@ -276,11 +307,10 @@ static cudaError_t karma_steps(pf_karma* k, int n)
         KarmaDesc d = k->d;
         d.it = k->it + 1;
         const int a = k->cur, b = 1 - k->cur;
-        k_karma_phase<T, kTY><<<grid, block, 0, k->stream>>>(d, c, (const T*)k->phi[a], (const T*)k->U[a],
-                                                             (T*)k->dphi, k->zchunk);
-        k_karma_solute<T, kTY><<<grid, block, 0, k->stream>>>(d, c, (const T*)k->phi[a], (const T*)k->U[a],
-                                                              (const T*)k->dphi, (T*)k->phi[b], (T*)k->U[b],
-                                                              k->zchunk);
+        k_karma_phase<T, kTY><<<grid, block, 0, k->stream>>>(k->tm_phi[a], d, c, (const T*)k->U[a], (T*)k->dphi,
+                                                             k->zchunk, k->d_status);
+        k_karma_solute<T, kTY><<<grid, block, 0, k->stream>>>(k->tm_phi[a], k->tm_u[a], k->tm_dphi, d, c,
+                                                              (T*)k->phi[b], (T*)k->U[b], k->zchunk, k->d_status);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) return e;
         k->cur = b;
@@ -308,19 +338,17 @@ int pf_karma_tip(pf_karma* k, int* tip_x, int* tip_d)
         k_karma_tip<float><<<1, 256, 0, k->stream>>>(k->d, (const float*)k->phi[k->cur], k->d_tip);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(k->h_tip, k->d_tip, 2 * sizeof(int), cudaMemcpyDeviceToHost, k->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(k->stream);
     if (e != cudaSuccess) return kerr(PF_E_CUDA, std::string("tip: ") + cudaGetErrorString(e));
+    const int rc = karma_wait(k, "tip");
     *tip_x = k->h_tip[0];
     *tip_d = k->h_tip[1];
-    return PF_OK;
+    return rc;
 }
 
 int pf_karma_sync(pf_karma* k)
 {
     if (!k) return kerr(PF_E_ARG, "null handle");
-    cudaError_t e = cudaStreamSynchronize(k->stream);
-    if (e != cudaSuccess) return kerr(PF_E_CUDA, std::string("sync: ") + cudaGetErrorString(e));
-    return PF_OK;
+    return karma_wait(k, "sync");
 }
 
 }  // extern "C"
