@@ -4,7 +4,8 @@
 // reference (principal.f90:61-63) in pitched FP64 or FP32 storage, one
 // stream, and the host scalars the reference keeps in module variables
 // (TP, M0, it, time).  The per-subroutine entry points launch the
-// one-thread-per-cell kernels; pf_step launches the fused z-marching passes.
+// z-marching passes that run one subroutine alone (the heat equation one
+// thread per cell); pf_step launches the fused z-marching passes.
 #include <cuda_runtime.h>
 #include <cmath>
 #include <cstdio>
@@ -78,7 +79,6 @@ struct pf_ctx {
     int nslot;               // PF_OPT_NSLOT: window mode of the march passes (0: 3)
     CUtensorMap tmap[2];     // tensor maps of the two phase-field buffers (32 x 8 march tiles)
     void* tmap_buf[2];       // their base addresses
-    int tmap_ok;
     int* d_status;           // kernel status word: 0, or the code a kernel left there
     std::vector<std::pair<cudaEvent_t, cudaEvent_t>> ev_first, ev_last;
     std::string err;
@@ -193,16 +193,16 @@ int pf_create(const pf_grid* g, const pf_params* p, int precision, pf_ctx** out)
         return set_global_err(PF_E_CUDA, std::string("context set-up: ") + cudaGetErrorString(e));
     }
     ctx->stream = ctx->own_stream;
-    // tensor maps of the phase-field buffers for the TMA plane loads; without
-    // them (driver entry point missing) the step uses the cp.async passes
+    // tensor maps of the phase-field buffers for the TMA plane loads
     ctx->kernel = 1;
     ctx->nslot = 0;
-    ctx->tmap_ok = 1;
     for (int b = 0; b < 2; ++b) {
         ctx->tmap_buf[b] = ctx->fld[b == 0 ? PF_PHASE_OLD : PF_PHASE_NEW];
         if (encode_field_map(&ctx->tmap[b], ctx->tmap_buf[b], (int)ctx->es, g->nx, g->ny, g->nz, px,
-                             march_box_x((int)ctx->es), march_box_y(8)) != 0)
-            ctx->tmap_ok = 0;
+                             march_box_x((int)ctx->es), march_box_y(8)) != 0) {
+            pf_destroy(ctx);
+            return set_global_err(PF_E_CUDA, "tensor map encoding failed");
+        }
     }
     *out = ctx;
     return PF_OK;
@@ -420,6 +420,32 @@ static Fields fields_of(const pf_ctx* ctx)
     return f;
 }
 
+// the tensor map of one of the two phase-field buffers
+static const CUtensorMap& tm_of(const pf_ctx* ctx, const void* buf)
+{
+    return ctx->tmap[buf == ctx->tmap_buf[0] ? 0 : 1];
+}
+
+// one phase sweep phi_in -> phi_out (dpp null: DPP is not written), and the
+// solute update c_in -> c_out, as kernels of their own
+static cudaError_t run_sweep(pf_ctx* ctx, const StepArgs& s, const void* phi_in, const void* c_in, void* phi_out,
+                             void* dpp)
+{
+    const int zc = ctx->zfill[is64(ctx) ? 0 : 1];
+    return is64(ctx) ? launch_march_sweep<double>(tm_of(ctx, phi_in), ctx->dd, s, c_in, phi_out, dpp, zc,
+                                                  ctx->d_status, ctx->stream)
+                     : launch_march_sweep<float>(tm_of(ctx, phi_in), ctx->dd, s, c_in, phi_out, dpp, zc,
+                                                 ctx->d_status, ctx->stream);
+}
+static cudaError_t run_solute(pf_ctx* ctx, const StepArgs& s, const void* phi_in, const void* c_in, void* c_out)
+{
+    const int zc = ctx->zfill[1];
+    return is64(ctx) ? launch_march_solute<double>(tm_of(ctx, phi_in), ctx->dd, s, c_in, c_out, zc, ctx->d_status,
+                                                   ctx->stream)
+                     : launch_march_solute<float>(tm_of(ctx, phi_in), ctx->dd, s, c_in, c_out, zc, ctx->d_status,
+                                                  ctx->stream);
+}
+
 int pf_temperatura(pf_ctx* ctx, double TP)
 {
     if (!ctx) return PF_E_ARG;
@@ -441,9 +467,7 @@ int pf_equacao_campo_fase(pf_ctx* ctx, int it, double TP, double M0, double* Cs_
     if (Cs_eq) *Cs_eq = Cs;
     if (Cl_eq) *Cl_eq = Cl;
     Fields f = fields_of(ctx);
-    CK(is64(ctx) ? launch_phase<double>(ctx->dd, s, f.phi_old, f.c_old, f.phi_new, f.dpp, ctx->stream)
-                 : launch_phase<float>(ctx->dd, s, f.phi_old, f.c_old, f.phi_new, f.dpp, ctx->stream),
-       "equacao_campo_fase");
+    CK(run_sweep(ctx, s, f.phi_old, f.c_old, f.phi_new, f.dpp), "equacao_campo_fase");
     return PF_OK;
 }
 
@@ -461,13 +485,10 @@ int pf_concentracao_soluto(pf_ctx* ctx)
     if (!ctx) return PF_E_ARG;
     StepArgs s = make_step_args(ctx->p, ctx->dv, ctx->st.it, ctx->st.TP, ctx->st.TP, ctx->st.M0);
     Fields f = fields_of(ctx);
-    if (is64(ctx)) {
-        CK(launch_solute<double>(ctx->dd, s, f.phi_old, f.c_old, f.c_new, ctx->stream), "concentracao_soluto");
-        CK(launch_copy_inner<double>(ctx->dd, f.c_new, f.c_old, ctx->stream), "concentracao_soluto old=new");
-    } else {
-        CK(launch_solute<float>(ctx->dd, s, f.phi_old, f.c_old, f.c_new, ctx->stream), "concentracao_soluto");
-        CK(launch_copy_inner<float>(ctx->dd, f.c_new, f.c_old, ctx->stream), "concentracao_soluto old=new");
-    }
+    CK(run_solute(ctx, s, f.phi_old, f.c_old, f.c_new), "concentracao_soluto");
+    CK(is64(ctx) ? launch_copy_inner<double>(ctx->dd, f.c_new, f.c_old, ctx->stream)
+                 : launch_copy_inner<float>(ctx->dd, f.c_new, f.c_old, ctx->stream),
+       "concentracao_soluto old=new");
     return PF_OK;
 }
 
@@ -659,7 +680,7 @@ static int one_step(pf_ctx* ctx)
     Fields f = fields_of(ctx);
     void* final_phi;
     void* other_phi;
-    const bool march = ctx->fused && ctx->kernel == 1 && ctx->tmap_ok && ctx->tile_y == 8;
+    const bool march = ctx->fused && ctx->kernel == 1 && ctx->tile_y == 8;
     if (march) {
         // TMA-staged passes: two cells per thread unless PF_OPT_PAIRED says
         // otherwise (default: FP32 only) or the deck draws the smooth noise
@@ -667,15 +688,12 @@ static int one_step(pf_ctx* ctx)
         const int nslot = ctx->nslot ? ctx->nslot : 3;
         const int occ_q = (is64(ctx) && p.ruido_tipo == 2) ? 0 : (lanes == 2 && !is64(ctx)) ? 2 : 1;
         const int zchunk = ctx->zchunk_set ? ctx->zchunk : ctx->zfill[occ_q];
-        auto tm_of = [ctx](const void* buf) -> const CUtensorMap& {
-            return ctx->tmap[buf == ctx->tmap_buf[0] ? 0 : 1];
-        };
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         f.phi_mid = B;
         if (ctx->ktiming) { e0 = new_event(); e1 = new_event(); cudaEventRecord(e0, ctx->stream); }
-        CK(is64(ctx) ? launch_march_first<double>(tm_of(A), ctx->dd, s, f, nsw == 1, lanes, nslot, zchunk,
+        CK(is64(ctx) ? launch_march_first<double>(tm_of(ctx, A), ctx->dd, s, f, nsw == 1, lanes, nslot, zchunk,
                                                   ctx->d_status, ctx->stream)
-                     : launch_march_first<float>(tm_of(A), ctx->dd, s, f, nsw == 1, lanes, nslot, zchunk,
+                     : launch_march_first<float>(tm_of(ctx, A), ctx->dd, s, f, nsw == 1, lanes, nslot, zchunk,
                                                  ctx->d_status, ctx->stream),
            nsw == 1 ? "march step (single sweep)" : "march heat + sweep 1");
         if (ctx->ktiming) { cudaEventRecord(e1, ctx->stream); ctx->ev_first.push_back({e0, e1}); }
@@ -687,18 +705,16 @@ static int one_step(pf_ctx* ctx)
             void* oth = A;   // free buffer
             for (int sw = 2; sw <= nsw - 1; ++sw) {
                 // no DPP: it carries the step's noise from the first to the last pass
-                CK(is64(ctx) ? launch_phase<double>(ctx->dd, s, cur, f.c_old, oth, nullptr, ctx->stream)
-                             : launch_phase<float>(ctx->dd, s, cur, f.c_old, oth, nullptr, ctx->stream),
-                   "middle sweep");
+                CK(run_sweep(ctx, s, cur, f.c_old, oth, nullptr), "middle sweep");
                 std::swap(cur, oth);
             }
             Fields f2 = f;
             f2.phi_mid = cur;
             f2.phi_new = oth;
             if (ctx->ktiming) { e0 = new_event(); e1 = new_event(); cudaEventRecord(e0, ctx->stream); }
-            CK(is64(ctx) ? launch_march_last<double>(tm_of(cur), ctx->dd, s, f2, lanes, nslot, zchunk,
+            CK(is64(ctx) ? launch_march_last<double>(tm_of(ctx, cur), ctx->dd, s, f2, lanes, nslot, zchunk,
                                                      ctx->d_status, ctx->stream)
-                         : launch_march_last<float>(tm_of(cur), ctx->dd, s, f2, lanes, nslot, zchunk,
+                         : launch_march_last<float>(tm_of(ctx, cur), ctx->dd, s, f2, lanes, nslot, zchunk,
                                                     ctx->d_status, ctx->stream),
                "march last sweep + solute");
             if (ctx->ktiming) { cudaEventRecord(e1, ctx->stream); ctx->ev_last.push_back({e0, e1}); }
@@ -735,9 +751,7 @@ static int one_step(pf_ctx* ctx)
             void* oth = A;   // free buffer
             for (int sw = 2; sw <= nsw - 1; ++sw) {
                 // no DPP: it carries the step's noise from the first to the last pass
-                CK(is64(ctx) ? launch_phase<double>(ctx->dd, s, cur, f.c_old, oth, nullptr, ctx->stream)
-                             : launch_phase<float>(ctx->dd, s, cur, f.c_old, oth, nullptr, ctx->stream),
-                   "middle sweep");
+                CK(run_sweep(ctx, s, cur, f.c_old, oth, nullptr), "middle sweep");
                 std::swap(cur, oth);
             }
             Fields f2 = f;
@@ -761,13 +775,9 @@ static int one_step(pf_ctx* ctx)
         void* out = B;
         for (int sw = 1; sw <= nsw; ++sw) {
             if (sw > 1) std::swap(in, out);   // the copy new -> old, by exchange
-            CK(is64(ctx) ? launch_phase<double>(ctx->dd, s, in, f.c_old, out, f.dpp, ctx->stream)
-                         : launch_phase<float>(ctx->dd, s, in, f.c_old, out, f.dpp, ctx->stream),
-               "equacao_campo_fase");
+            CK(run_sweep(ctx, s, in, f.c_old, out, f.dpp), "equacao_campo_fase");
         }
-        CK(is64(ctx) ? launch_solute<double>(ctx->dd, s, in, f.c_old, f.c_new, ctx->stream)
-                     : launch_solute<float>(ctx->dd, s, in, f.c_old, f.c_new, ctx->stream),
-           "concentracao_soluto");
+        CK(run_solute(ctx, s, in, f.c_old, f.c_new), "concentracao_soluto");
         final_phi = out;
         other_phi = in;
     }

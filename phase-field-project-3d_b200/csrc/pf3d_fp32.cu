@@ -9,8 +9,6 @@
 
 namespace pf3d {
 template cudaError_t launch_heat<float>(const DomainDesc&, const StepArgs&, const Fields&, cudaStream_t);
-template cudaError_t launch_phase<float>(const DomainDesc&, const StepArgs&, const void*, const void*, void*, void*, cudaStream_t);
-template cudaError_t launch_solute<float>(const DomainDesc&, const StepArgs&, const void*, const void*, void*, cudaStream_t);
 template cudaError_t launch_copy_inner<float>(const DomainDesc&, const void*, void*, cudaStream_t);
 template cudaError_t launch_fused_first<float>(const DomainDesc&, const StepArgs&, const Fields&, bool, int, int, cudaStream_t);
 template cudaError_t launch_fused_last<float>(const DomainDesc&, const StepArgs&, const Fields&, int, int, cudaStream_t);

@@ -1,4 +1,4 @@
-// pf3d_fp64.cu -- FP64 per-subroutine kernels (reference form), diagnostics and
+// pf3d_fp64.cu -- FP64 heat and copy kernels (reference form), diagnostics and
 // staging conversions.
 // Built with --fmad=false: the reference's gfortran arithmetic on x86-64 has
 // no fused multiply-add, so neither may this form.
@@ -9,8 +9,6 @@
 
 namespace pf3d {
 template cudaError_t launch_heat<double>(const DomainDesc&, const StepArgs&, const Fields&, cudaStream_t);
-template cudaError_t launch_phase<double>(const DomainDesc&, const StepArgs&, const void*, const void*, void*, void*, cudaStream_t);
-template cudaError_t launch_solute<double>(const DomainDesc&, const StepArgs&, const void*, const void*, void*, cudaStream_t);
 template cudaError_t launch_copy_inner<double>(const DomainDesc&, const void*, void*, cudaStream_t);
 template cudaError_t launch_diag<double>(const DomainDesc&, const void*, const void*, const void*, const void*, double*, int, double*, cudaStream_t);
 template cudaError_t launch_convert_in<double>(const DomainDesc&, const double*, void*, long long, long long, cudaStream_t);

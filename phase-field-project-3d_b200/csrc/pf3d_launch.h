@@ -20,12 +20,9 @@ struct Fields {
     void* phi_mid;   // fused step: the sweep-1 phase field
 };
 
-// Per-subroutine kernels (one thread per cell, reference form).
+// One-thread-per-cell subroutine kernels: temperatura, and the interior copy
+// of concentracao_soluto.
 template <typename T> cudaError_t launch_heat(const DomainDesc& d, const StepArgs& s, const Fields& f, cudaStream_t st);
-template <typename T> cudaError_t launch_phase(const DomainDesc& d, const StepArgs& s, const void* phi_in,
-                                               const void* c_in, void* phi_out, void* dpp, cudaStream_t st);
-template <typename T> cudaError_t launch_solute(const DomainDesc& d, const StepArgs& s, const void* phi_in,
-                                                const void* c_in, void* c_out, cudaStream_t st);
 template <typename T> cudaError_t launch_copy_inner(const DomainDesc& d, const void* src, void* dst, cudaStream_t st);
 
 // Fused z-marching kernels.
@@ -85,6 +82,14 @@ template <typename S> cudaError_t launch_march_first(const CUtensorMap& tm, cons
 template <typename S> cudaError_t launch_march_last(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s,
                                                     const Fields& f, int lanes, int nslot, int zchunk, int* err,
                                                     cudaStream_t st);
+// one subroutine alone (FP64: reference form): a phase sweep (dpp may be null)
+// and the solute update
+template <typename S> cudaError_t launch_march_sweep(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s,
+                                                     const void* c_in, void* phi_out, void* dpp, int zchunk, int* err,
+                                                     cudaStream_t st);
+template <typename S> cudaError_t launch_march_solute(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s,
+                                                      const void* c_in, void* c_out, int zchunk, int* err,
+                                                      cudaStream_t st);
 // batch form: tmaps[2 d + b] is the tensor map of buffer b of domain d's
 // phase field; *ctr (zero before the launch) hands out the work items
 template <typename S> cudaError_t launch_march_batch(const BatchDomain* doms, const CUtensorMap* tmaps,

@@ -76,7 +76,7 @@ template <int WIN> struct MarchWin {
 };
 
 // Shared-memory layout of one tile (bytes from a 128-byte aligned base).
-template <typename S, int TY, bool SOL, int NSLOT>
+template <typename S, int TY, bool SOL, int NSLOT, bool PHASE = true, bool FAST = true>
 struct MarchLayout {
     static constexpr int TX = 32;
     // the TMA box starts XOFF cells left of the tile: x * sizeof(S) must be a
@@ -93,8 +93,8 @@ struct MarchLayout {
     static constexpr int BAR_OFF = NPHI * PHI_BYTES;
     static constexpr int NODE_OFF = (BAR_OFF + NPHI * 8 + 127) / 128 * 128;
     static constexpr int NODE_SLOT = 4 * NQ;       // eps^2, exy, eyz, ezx
-    static constexpr int SOL_OFF = NODE_OFF + NSLOT * NODE_SLOT * (int)sizeof(S);
-    static constexpr int SOL_SLOT = 2 * NQ;        // Gamma bracket, mu
+    static constexpr int SOL_OFF = NODE_OFF + (PHASE ? NSLOT * NODE_SLOT * (int)sizeof(S) : 0);
+    static constexpr int SOL_SLOT = (FAST ? 2 : 3) * NQ;   // Gamma bracket, mu; reference form 1/GAMMA twice, mu
     static constexpr int BYTES = SOL_OFF + (SOL ? NSLOT * SOL_SLOT * (int)sizeof(S) : 0);
     static constexpr int ALLOC = BYTES + 128;      // slack to align the dynamic base
 };
@@ -133,10 +133,9 @@ __device__ __forceinline__ unsigned char* align128(unsigned char* p)
 
 // Initialises the six plane barriers of a tile's window (one thread), made
 // visible to the TMA unit and to every thread of the CTA.
-template <typename S, int TY, bool SOL, int NSLOT>
+template <typename LY>
 __device__ __forceinline__ void march_init_barriers(unsigned char* smem)
 {
-    using LY = MarchLayout<S, TY, SOL, NSLOT>;
     if (threadIdx.x == 0 && threadIdx.y == 0) {
         const uint32_t b0 = smem_u32(smem + LY::BAR_OFF);
         for (int s = 0; s < LY::NPHI; ++s) mbar_init(b0 + 8 * s, 1);
@@ -151,8 +150,11 @@ __device__ __forceinline__ void march_init_barriers(unsigned char* smem)
 // issued is waited for).  Returns false if a plane load did not arrive in
 // time; the CTA must then stop.  SPLIT: a second copy of the plane body for
 // the interior planes, without their z checks (single domains; a batch's
-// short items gain less than the larger code costs them, measured).
-template <typename S, int L, int TY, int WIN, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool SPLIT = true>
+// short items gain less than the larger code costs them, measured).  PHASE =
+// false leaves the phase sweep out (the solute subroutine alone); FAST = false
+// is the reference form of the per-subroutine entry points (FP64, one lane).
+template <typename S, int L, int TY, int WIN, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool SPLIT = true,
+          bool PHASE = true, bool FAST = true>
 __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, const KC<typename Lanes<S, L>::V>& cv,
                                            const CUtensorMap* tm, const S* __restrict__ c_in,
                                            S* __restrict__ phi_out, S* __restrict__ dpp, S* __restrict__ c_out,
@@ -163,10 +165,10 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
     using V = typename LN::V;
     constexpr int NSLOT = MarchWin<WIN>::nslot;
     constexpr bool ROLL = MarchWin<WIN>::roll;
-    using LY = MarchLayout<S, TY, SOL, NSLOT>;
+    using LY = MarchLayout<S, TY, SOL, NSLOT, PHASE, FAST>;
     constexpr int TX = 32, TW = LY::TW, NW = LY::NW, NH = LY::NH, NQ = LY::NQ, XOFF = LY::XOFF;
     constexpr int TR = TY / L;                                    // thread rows; lane l owns row ty + l*TR
-    constexpr int ran_mode = (HEAT && !DPPW) ? 1 : ((!HEAT && DPPW) ? 2 : 0);
+    constexpr int ran_mode = (HEAT && !DPPW) ? 1 : ((!HEAT && DPPW && SOL) ? 2 : 0);
     constexpr int NRING = (L == 1) ? 2 * NW + 2 * TY : NW + TY;  // ring items (pairs when L = 2)
     static_assert(TY % L == 0, "tile height must be a multiple of the lanes");
 
@@ -259,7 +261,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
     // the node quantities of one set of items from their gradient; stored
     // into the slot `dst`; the own items' eps^2, eyz, ezx also into `keep`
     auto node_store = [&](S* dst, const int* off_node, V gx, V gy, V gz, S (*keep)[3]) {
-        const Node<V> q = aniso_node<V, true>(gx, gy, gz, cv);
+        const Node<V> q = aniso_node<V, FAST>(gx, gy, gz, cv);
         const V eps2 = q.eps * q.eps;   // the stencil reads eps only squared
 #pragma unroll
         for (int l = 0; l < L; ++l) {
@@ -283,13 +285,13 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
             S a[L], b[L];
 #pragma unroll
             for (int l = 0; l < L; ++l) { a[l] = p0[off_phi[l] + 1]; b[l] = p0[off_phi[l] - 1]; }
-            const V gx = grad<V, true>(LN::make(a), LN::make(b), cv.dx, cv.hx);
+            const V gx = grad<V, FAST>(LN::make(a), LN::make(b), cv.dx, cv.hx);
 #pragma unroll
             for (int l = 0; l < L; ++l) { a[l] = p0[off_phi[l] + TW]; b[l] = p0[off_phi[l] - TW]; }
-            const V gy = grad<V, true>(LN::make(a), LN::make(b), cv.dy, cv.hy);
+            const V gy = grad<V, FAST>(LN::make(a), LN::make(b), cv.dy, cv.hy);
 #pragma unroll
             for (int l = 0; l < L; ++l) { a[l] = pp[off_phi[l]]; b[l] = pm[off_phi[l]]; }
-            const V gz = grad<V, true>(LN::make(a), LN::make(b), cv.dz, cv.hz);
+            const V gz = grad<V, FAST>(LN::make(a), LN::make(b), cv.dz, cv.hz);
             node_store(dst, off_node, gx, gy, gz, kp);
         };
         one(phi_off, node_off, keep);
@@ -305,12 +307,13 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
             S a[L];
 #pragma unroll
             for (int l = 0; l < L; ++l) a[l] = op ? op[l] : p0[off_phi[l]];
-            const SolNode<V> q = sol_node<V, true>(LN::make(a), LN::make(cc), cv);
+            const SolNode<V> q = sol_node<V, FAST>(LN::make(a), LN::make(cc), cv);
 #pragma unroll
             for (int l = 0; l < L; ++l) {
                 S* o = dst + off_node[l];
-                o[0] = LN::get(q.br, l);
+                o[0] = LN::get(FAST ? q.br : q.il, l);
                 o[NQ] = LN::get(q.mu, l);
+                if (!FAST) o[2 * NQ] = LN::get(q.is, l);
                 if (kp) {
                     kp[l][0] = LN::get(q.br, l);
                     kp[l][1] = LN::get(q.mu, l);
@@ -412,11 +415,11 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
             if (p >= 0 && p <= zlast) bad |= !wait_plane((p + 6) % 6);
     }
     load_centre(zb);
-    if (zb - 1 >= 1 && zb - 1 <= nz - 2)
+    if (PHASE && zb - 1 >= 1 && zb - 1 <= nz - 2)
         node_plane(wrap_add<NSLOT>(zb % NSLOT, NSLOT - 1), sphi + ((zb + 4) % 6) * LY::PHI_SLOT,
                    sphi + ((zb + 5) % 6) * LY::PHI_SLOT,
                    sphi + (zb % 6) * LY::PHI_SLOT, ROLL ? rnB : nullptr);
-    if (zb >= 1 && zb <= nz - 2)
+    if (PHASE && zb >= 1 && zb <= nz - 2)
         node_plane(zb % NSLOT, sphi + ((zb + 5) % 6) * LY::PHI_SLOT, sphi + (zb % 6) * LY::PHI_SLOT,
                    sphi + ((zb + 1) % 6) * LY::PHI_SLOT, ROLL ? rnC : nullptr);
     load5(rpm, sphi + ((zb + 5) % 6) * LY::PHI_SLOT);
@@ -460,25 +463,25 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
                 S a[L], b[L];
 #pragma unroll
                 for (int l = 0; l < L; ++l) { a[l] = rpp[l][3]; b[l] = rpp[l][4]; }
-                const V gx = grad<V, true>(LN::make(a), LN::make(b), cv.dx, cv.hx);
+                const V gx = grad<V, FAST>(LN::make(a), LN::make(b), cv.dx, cv.hx);
 #pragma unroll
                 for (int l = 0; l < L; ++l) { a[l] = rpp[l][1]; b[l] = rpp[l][2]; }
-                const V gy = grad<V, true>(LN::make(a), LN::make(b), cv.dy, cv.hy);
+                const V gy = grad<V, FAST>(LN::make(a), LN::make(b), cv.dy, cv.hy);
 #pragma unroll
                 for (int l = 0; l < L; ++l) { a[l] = pq[phi_off[l]]; b[l] = rp0[l][0]; }
-                const V gz = grad<V, true>(LN::make(a), LN::make(b), cv.dz, cv.hz);
+                const V gz = grad<V, FAST>(LN::make(a), LN::make(b), cv.dz, cv.hz);
                 S* const dst = snode + snp1 * LY::NODE_SLOT;
                 node_store(dst, node_off, gx, gy, gz, rnT);
                 if (ring) {
 #pragma unroll
                     for (int l = 0; l < L; ++l) { a[l] = pp[rphi_off[l] + 1]; b[l] = pp[rphi_off[l] - 1]; }
-                    const V rx = grad<V, true>(LN::make(a), LN::make(b), cv.dx, cv.hx);
+                    const V rx = grad<V, FAST>(LN::make(a), LN::make(b), cv.dx, cv.hx);
 #pragma unroll
                     for (int l = 0; l < L; ++l) { a[l] = pp[rphi_off[l] + TW]; b[l] = pp[rphi_off[l] - TW]; }
-                    const V ry = grad<V, true>(LN::make(a), LN::make(b), cv.dy, cv.hy);
+                    const V ry = grad<V, FAST>(LN::make(a), LN::make(b), cv.dy, cv.hy);
 #pragma unroll
                     for (int l = 0; l < L; ++l) { a[l] = pq[rphi_off[l]]; b[l] = p0[rphi_off[l]]; }
-                    const V rz = grad<V, true>(LN::make(a), LN::make(b), cv.dz, cv.hz);
+                    const V rz = grad<V, FAST>(LN::make(a), LN::make(b), cv.dz, cv.hz);
                     node_store(dst, rnode_off, rx, ry, rz, nullptr);
                 }
             }
@@ -489,7 +492,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
                 sol_plane(snp1, pp, co[1], cr[0], rsT, op);
             }
         } else {
-            if (IN || (z + 1 >= 1 && z + 1 <= nz - 2)) node_plane(snp1, p0, pp, pq, nullptr);
+            if (PHASE && (IN || (z + 1 >= 1 && z + 1 <= nz - 2))) node_plane(snp1, p0, pp, pq, nullptr);
             if (SOL && (IN || z + 1 <= nz - 1)) sol_plane(snp1, pp, co[1], cr[0], nullptr, nullptr);
         }
         // D: one barrier orders the plane; everyone learns of a failed load
@@ -519,7 +522,9 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
         float ran[L];
 #pragma unroll
         for (int l = 0; l < L; ++l) {
-            if constexpr (ran_mode == 2) {
+            if constexpr (!PHASE) {
+                ran[l] = 0.f;
+            } else if constexpr (ran_mode == 2) {
                 ran[l] = (float)dcur[l];
             } else if constexpr (SMOOTH) {
                 ran[l] = (c.rt == 2) ? phase_ran(2, x + 1, yv[l] + 1, z + 1, c.it)
@@ -531,7 +536,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
         }
 
         V ppn = PP;
-        if (zph) {
+        if (PHASE && zph) {
             Nbr<V> nb;
             S t[L];
 #define PF3D_NB(FIELD, PLANE, DELTA)                                         \
@@ -579,7 +584,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
             S rs[L];
 #pragma unroll
             for (int l = 0; l < L; ++l) rs[l] = (S)ran[l];
-            ppn = phase_ppnew<V, true, true>(nb, E, W, N, So, Tt, B, CPP, LN::make(rs), cv);
+            ppn = phase_ppnew<V, FAST, true>(nb, E, W, N, So, Tt, B, CPP, LN::make(rs), cv);
         }
         V cn = CPP;
         if (SOL && zin) {
@@ -591,8 +596,12 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
 #define PF3D_SN(I, PLANE, DELTA)                                                                   \
     _Pragma("unroll") for (int l = 0; l < L; ++l) { a[l] = PLANE[node_off[l] + (DELTA)];          \
                                                      b[l] = PLANE[node_off[l] + (DELTA) + NQ]; }  \
-    q[I].br = LN::make(a);                                                                         \
-    q[I].mu = LN::make(b);
+    q[I].br = q[I].il = LN::make(a);                                                               \
+    q[I].mu = LN::make(b);                                                                         \
+    if constexpr (!FAST) {                                                                         \
+        _Pragma("unroll") for (int l = 0; l < L; ++l) a[l] = PLANE[node_off[l] + (DELTA) + 2 * NQ]; \
+        q[I].is = LN::make(a);                                                                     \
+    }
             PF3D_SN(1, s0, 1) PF3D_SN(2, s0, -1) PF3D_SN(3, s0, NW) PF3D_SN(4, s0, -NW)
             if constexpr (ROLL) {
 #define PF3D_SR(I, ARR)                                                                              \
@@ -605,7 +614,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
                 PF3D_SN(0, s0, 0) PF3D_SN(5, sp1, 0) PF3D_SN(6, sm1, 0)
             }
 #undef PF3D_SN
-            cn = conc_new<V, true>(PP, CPP, q[0], q[1], q[2], q[3], q[4], q[5], q[6], cv);
+            cn = conc_new<V, FAST>(PP, CPP, q[0], q[1], q[2], q[3], q[4], q[5], q[6], cv);
         }
         const V U = clamp01(ppn);
         const V DP = ppn - PP;
@@ -619,7 +628,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
                 if (HEAT) T_new[id] = heat_at<S>(T_old, id, px, pl, PPs[l], dcur[l], c);
                 if (ran_mode == 1) dpp[id] = (S)ran[l];
                 if (DPPW) dpp[id] = LN::get(DP, l);
-                phi_out[id] = LN::get(U, l);
+                if (PHASE) phi_out[id] = LN::get(U, l);
                 if (SOL) c_out[id] = LN::get(cn, l);
             }
         } else {
@@ -634,7 +643,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
                     if (src) tn = heat_at<S>(T_old, id, px, pl, PPs[l], dcur[l], c);
                     T_new[id] = tn;
                 }
-                if (src) {
+                if (PHASE && src) {
                     const bool inner = xph && yph[l] && zph;
                     S u = PPs[l];
                     if (inner) {
@@ -732,8 +741,9 @@ struct MarchOcc {
 };
 
 // single domain: one CTA per tile; the phase field comes through `tm`
-template <typename S, int L, int TY, int WIN, bool HEAT, bool DPPW, bool SOL, bool SMOOTH>
-__global__ void __launch_bounds__(32 * TY / L, (MarchOcc<S, L, WIN, SOL, HEAT, SMOOTH>::v))
+template <typename S, int L, int TY, int WIN, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool PHASE = true,
+          bool FAST = true>
+__global__ void __launch_bounds__(32 * TY / L, (FAST ? MarchOcc<S, L, WIN, SOL, HEAT, SMOOTH>::v : PHASE ? 2 : 3))
     k_march(const __grid_constant__ CUtensorMap tm, DomainDesc d, const KC<S> c,
             const KC<typename Lanes<S, L>::V> cv, const S* __restrict__ c_in, S* __restrict__ phi_out,
             S* __restrict__ dpp, S* __restrict__ c_out, const S* __restrict__ T_old, S* __restrict__ T_new,
@@ -741,9 +751,9 @@ __global__ void __launch_bounds__(32 * TY / L, (MarchOcc<S, L, WIN, SOL, HEAT, S
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* smem = align128(smem_raw);
-    march_init_barriers<S, TY, SOL, MarchWin<WIN>::nslot>(smem);
+    march_init_barriers<MarchLayout<S, TY, SOL, MarchWin<WIN>::nslot, PHASE, FAST>>(smem);
     uint32_t par = 0;
-    if (!march_tile<S, L, TY, WIN, HEAT, DPPW, SOL, SMOOTH>(d, c, cv, &tm, c_in, phi_out, dpp, c_out, T_old,
+    if (!march_tile<S, L, TY, WIN, HEAT, DPPW, SOL, SMOOTH, true, PHASE, FAST>(d, c, cv, &tm, c_in, phi_out, dpp, c_out, T_old,
                                                                 T_new, zchunk, blockIdx.x, blockIdx.y, blockIdx.z,
                                                                 smem, par)) {
         if (threadIdx.x == 0 && threadIdx.y == 0) atomicExch(err, kErrTmaTimeout);
@@ -774,7 +784,7 @@ __global__ void __launch_bounds__(32 * TY / L,
     constexpr int nf = (int)(offsetof(KC<S>, hq) / sizeof(S));
     constexpr int NT = 32 * TY / L;
     unsigned char* smem = align128(smem_raw);
-    march_init_barriers<S, TY, SOL, MarchWin<WIN>::nslot>(smem);
+    march_init_barriers<MarchLayout<S, TY, SOL, MarchWin<WIN>::nslot>>(smem);
     uint32_t par = 0;
     const int n = *n_items;
     const int tid = threadIdx.x + 32 * threadIdx.y;
@@ -860,13 +870,14 @@ KC<typename Lanes<S, L>::V> kc_lanes(const KC<S>& k)
     }
 }
 
-template <typename S, int L, int TY, int WIN, bool HEAT, bool DPPW, bool SOL, bool SMOOTH>
+template <typename S, int L, int TY, int WIN, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool PHASE = true,
+          bool FAST = true>
 cudaError_t launch_march_t(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s, const void* c_in,
                            void* phi_out, void* dpp, void* c_out, const void* T_old, void* T_new, int zchunk,
                            int* err, cudaStream_t st)
 {
-    using LY = MarchLayout<S, TY, SOL, MarchWin<WIN>::nslot>;
-    auto kern = k_march<S, L, TY, WIN, HEAT, DPPW, SOL, SMOOTH>;
+    using LY = MarchLayout<S, TY, SOL, MarchWin<WIN>::nslot, PHASE, FAST>;
+    auto kern = k_march<S, L, TY, WIN, HEAT, DPPW, SOL, SMOOTH, PHASE, FAST>;
     static bool configured = false;   // one attribute call per instantiation
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::ALLOC);
@@ -914,6 +925,34 @@ cudaError_t launch_march_last(const CUtensorMap& tm, const DomainDesc& d, const 
     return lanes == 2 ? PF3D_MW(2) : PF3D_MW(1);
 #undef PF3D_MW
 #undef PF3D_ML
+}
+
+// One subroutine alone, for the per-subroutine entry points and the middle
+// sweeps of a step with more than two: equacao_campo_fase (dpp null: DPP is
+// not written) and concentracao_soluto without its copy to conc_soluto_old.
+// FP64 runs the reference form, FP32 the fast form; every node's and point's
+// quantities are computed once and shared, where one thread per cell computed
+// six nodes and seven points a cell.  128x128x256 FP64: a whole step of
+// subroutine calls 1146 -> 453 us (a sweep 430 -> 149 us, the solute step with
+// its copy 230 -> 115 us; with the general divisions the sweep took 336 us).
+template <typename S>
+cudaError_t launch_march_sweep(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s, const void* c_in,
+                               void* phi_out, void* dpp, int zchunk, int* err, cudaStream_t st)
+{
+    constexpr bool FAST = sizeof(S) == 4;
+    const bool smooth = d.rt == 2;
+#define PF3D_MS(DW, SM)                                                                                                 launch_march_t<S, 1, 8, 3, false, DW, false, SM, true, FAST>(tm, d, s, c_in, phi_out, dpp, nullptr, nullptr,                                                                     nullptr, zchunk, err, st)
+    if (dpp) return smooth ? PF3D_MS(true, true) : PF3D_MS(true, false);
+    return smooth ? PF3D_MS(false, true) : PF3D_MS(false, false);
+#undef PF3D_MS
+}
+
+template <typename S>
+cudaError_t launch_march_solute(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s, const void* c_in,
+                                void* c_out, int zchunk, int* err, cudaStream_t st)
+{
+    return launch_march_t<S, 1, 8, 3, false, false, true, false, false, sizeof(S) == 4>(
+        tm, d, s, c_in, nullptr, nullptr, c_out, nullptr, nullptr, zchunk, err, st);
 }
 
 // The persistent grid is the SM count times the CTAs of this kernel that are
