@@ -322,8 +322,11 @@ int pf_batch_step_async(pf_batch* b, int n_steps);
 int pf_batch_wait(pf_batch* b);
 /* device milliseconds of the last pf_batch_step call (all its graphs)      */
 double pf_batch_last_ms(const pf_batch* b);
+/* tile height and z-chunk; until set (or autotuned) tiles are 32 x 8 and the
+   TMA passes take the chunk that suits the batch's membership               */
 int pf_batch_set_tile(pf_batch* b, int tile_y, int zchunk);
-/* 32 x 8 tiles: 1 runs two cells per thread (same results), 0 one.  The
+/* 32 x 8 tiles: 1 runs two cells per thread (same results), 0 one; until set,
+   two in FP32 batches on the TMA passes, else one.  The
    TMA passes pair cells in either precision, except in batches with the
    smooth noise; the cp.async passes pair FP32 batches without the smooth
    noise or heat diffusion only                                             */

@@ -82,7 +82,9 @@ struct pf_batch {
     double* h_out = nullptr;
     double* d_sites = nullptr;         // bump sites for device initialisation
     int tile_y = 8, zchunk = 64, n_sm = 0;   // persistent grids: n_sm x resident CTAs
-    int pair = 0;                      // 32 x 8 tiles with two cells per thread (set by the autotuner)
+    bool zauto = true;                 // the chunk follows the membership (batch_zchunk) until a tile is set
+    int zc = 64;                       // chunk of the current work list
+    int pair = -1;                     // 32 x 8 tiles with two cells per thread; -1: FP32 yes, FP64 no
     int march = 1;                     // TMA-staged march passes (32 x 8 tiles); 0: the cp.async passes
     int nslot = 0;                     // window mode of the march passes (0: 3)
     CUtensorMap* d_tmaps = nullptr;    // 2 per slot: the tensor maps of its phase-field buffers
@@ -113,8 +115,48 @@ static int berr(pf_batch* b, int code, const std::string& msg)
 
 static bool b64(const pf_batch* b) { return b->prec == PF_FP64; }
 
+// two cells per thread on 32 x 8 tiles: as set, or as the single-domain passes
+// default to (FP32, where it is faster: 12 domains of 32 .. 128 cells across,
+// 704 -> 608 us a step at the same chunk)
+static bool want_pair(const pf_batch* b) { return b->pair < 0 ? !b64(b) : b->pair != 0; }
+
+// Planes per z-chunk of the TMA passes for the current membership.  A CTA
+// works through items of `zc` planes, each with a prologue of about three
+// planes' work; long chunks leave CTAs idle at the end (about one chunk), or
+// from the start when there are fewer items than resident CTAs.  The chunk
+// with the least modelled time wins.  Measured on those 12 domains (FP32,
+// paired): 623 / 608 / 657 / 912 us a step at 8 / 16 / 32 / 64 planes, modelled
+// 95 / 92 / 102 / 131; batches of hundreds of millions of cells keep 64.
+static int batch_zchunk(const pf_batch* b)
+{
+    const int occ = want_pair(b) && !b64(b) ? 6 : 3;
+    const double slots = (double)b->n_sm * occ;
+    int best_zc = 64;
+    double best = 1e300;
+    for (int zc : {1, 2, 3, 4, 5, 6, 8, 10, 12, 16, 20, 24, 32, 48, 64}) {
+        double items = 0.0, planes = 0.0;
+        for (const Slot& sl : b->slots) {
+            if (!sl.used) continue;
+            const double t = (double)((sl.g.nx + 31) / 32) * ((sl.g.ny + 7) / 8), n = (sl.g.nz + zc - 1) / zc;
+            items += t * n;
+            planes += t * (sl.g.nz + 3.0 * n);
+        }
+        double t;
+        if (items <= slots) t = (1.0 + 0.14 * (std::ceil(items / b->n_sm) - 1.0)) * (zc + 3.0);
+        else t = (1.0 + 0.14 * (occ - 1)) * (planes / slots + zc + 3.0);
+        if (t < best) {
+            best = t;
+            best_zc = zc;
+        }
+    }
+    return best_zc;
+}
+
+static bool use_march(const pf_batch* b) { return b->march && b->tile_y == 8; }
+
 static int rebuild_items(pf_batch* b)
 {
+    b->zc = b->zauto && use_march(b) ? batch_zchunk(b) : b->zchunk;
     std::vector<BatchItem> items;
     // largest domains first: their items are the longest-running
     std::vector<int> order;
@@ -128,7 +170,7 @@ static int rebuild_items(pf_batch* b)
     for (int s : order) {
         const pf_grid& g = b->slots[s].g;
         const int nbx = (g.nx + 31) / 32, nby = (g.ny + b->tile_y - 1) / b->tile_y;
-        const int nbz = (g.nz + b->zchunk - 1) / b->zchunk;
+        const int nbz = (g.nz + b->zc - 1) / b->zc;
         for (int bz = 0; bz < nbz; ++bz)
             for (int by = 0; by < nby; ++by)
                 for (int bx = 0; bx < nbx; ++bx) items.push_back(BatchItem{s, bx, by, bz});
@@ -146,7 +188,8 @@ static int rebuild_items(pf_batch* b)
     }
     if (n) BCK(cudaMemcpyAsync(b->d_items, items.data(), n * sizeof(BatchItem), cudaMemcpyHostToDevice, b->stream),
                "work list upload");
-    BCK(cudaMemcpyAsync(b->d_nitems, &n, sizeof(int), cudaMemcpyHostToDevice, b->stream), "work list size");
+    const int head[2] = {n, b->zc};
+    BCK(cudaMemcpyAsync(b->d_nitems, head, sizeof(head), cudaMemcpyHostToDevice, b->stream), "work list size");
     BCK(cudaStreamSynchronize(b->stream), "work list sync");   // the host vector goes out of scope
     b->items_dirty = false;
     return PF_OK;
@@ -169,20 +212,19 @@ static bool any_lap(const pf_batch* b)
     return false;
 }
 
-static bool use_march(const pf_batch* b) { return b->march && b->tile_y == 8; }
-
 static int capture_graph(pf_batch* b)
 {
     const bool smooth = any_smooth(b);
     const bool march = use_march(b);
     const int nslot = b->nslot ? b->nslot : 3;
-    // two cells per thread on 32 x 8 tiles when the autotuner measured it
-    // faster: the march passes in either precision (not with the smooth
-    // noise); the cp.async passes in FP32 only, on decks without heat
-    // diffusion (their boundary tiles run the one-cell code twice)
-    const bool pair = march ? (b->pair && !smooth)
-                            : (b->pair && !b64(b) && b->tile_y == 8 && !smooth && !any_lap(b));
-    if (b->graph && b->graph_ty == b->tile_y && b->graph_zc == b->zchunk && b->graph_nsm == b->n_sm &&
+    // two cells per thread on 32 x 8 tiles: the march passes in either
+    // precision (not with the smooth noise); the cp.async passes where it was
+    // asked for, in FP32 only, on decks without heat diffusion (their boundary
+    // tiles run the one-cell code twice)
+    const bool pair = march ? (want_pair(b) && !smooth)
+                            : (b->pair == 1 && !b64(b) && b->tile_y == 8 && !smooth && !any_lap(b));
+    const int zc = march ? 0 : b->zchunk;   // the march passes read their chunk from the work list's head
+    if (b->graph && b->graph_ty == b->tile_y && b->graph_zc == zc && b->graph_nsm == b->n_sm &&
         b->graph_nsw == b->nsw && b->graph_smooth == smooth && b->graph_pair == pair &&
         b->graph_march == (int)march && b->graph_nslot == nslot)
         return PF_OK;
@@ -204,11 +246,11 @@ static int capture_graph(pf_batch* b)
                 const int lanes = pair ? 2 : 1;
                 for (int pass = 0; pass <= (one ? 0 : 1) && e == cudaSuccess; ++pass)
                     e = b64(b) ? launch_march_batch<double>(b->d_doms, b->d_tmaps, st, b->d_items, b->d_nitems, pass,
-                                                            one, smooth && pass == 0, lanes, nslot, b->zchunk,
-                                                            b->n_sm, b->d_ctr + 2 * k + pass, b->d_status, cs)
+                                                            one, smooth && pass == 0, lanes, nslot, b->n_sm,
+                                                            b->d_ctr + 2 * k + pass, b->d_status, cs)
                                : launch_march_batch<float>(b->d_doms, b->d_tmaps, st, b->d_items, b->d_nitems, pass,
-                                                           one, smooth && pass == 0, lanes, nslot, b->zchunk,
-                                                           b->n_sm, b->d_ctr + 2 * k + pass, b->d_status, cs);
+                                                           one, smooth && pass == 0, lanes, nslot, b->n_sm,
+                                                           b->d_ctr + 2 * k + pass, b->d_status, cs);
                 continue;
             }
             if (pair) {
@@ -237,7 +279,7 @@ static int capture_graph(pf_batch* b)
     cudaStreamDestroy(cs);
     if (e != cudaSuccess) return berr(b, PF_E_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
     b->graph_ty = b->tile_y;
-    b->graph_zc = b->zchunk;
+    b->graph_zc = zc;
     b->graph_nsm = b->n_sm;
     b->graph_nsw = b->nsw;
     b->graph_smooth = smooth;
@@ -256,16 +298,17 @@ static int set_grid(pf_batch* b)
     return PF_OK;
 }
 
-// Fills step table rows for up to kGraphSteps steps; returns how many steps
-// any slot advances.  Advances each slot's host state like pf_step does.
-static int fill_steps(pf_batch* b, BatchStep* rows, int nsteps)
+// Fills step table rows for up to kGraphSteps steps of slots 0 .. n_rows-1 (the
+// slots the work list names; the rows of a step are n_rows apart here);
+// returns how many steps any slot advances.  Advances each slot's host state
+// like pf_step does.
+static int fill_steps(pf_batch* b, BatchStep* rows, int nsteps, int n_rows)
 {
     int advanced = 0;
-    std::memset(rows, 0, sizeof(BatchStep) * (size_t)kGraphSteps * b->max_domains);
     for (int k = 0; k < kGraphSteps; ++k) {
-        for (int sidx = 0; sidx < (int)b->slots.size(); ++sidx) {
+        for (int sidx = 0; sidx < n_rows; ++sidx) {
             Slot& sl = b->slots[sidx];
-            BatchStep& r = rows[(size_t)k * b->max_domains + sidx];
+            BatchStep& r = rows[(size_t)k * n_rows + sidx];
             r.active = 0;
             if (!sl.used || k >= nsteps) continue;
             if (sl.target > 0 && sl.st.it >= sl.target) continue;
@@ -333,7 +376,7 @@ int pf_batch_create(int precision, long long budget_bytes, int max_domains, pf_b
         (e = cudaMalloc(&b->d_steps, step_bytes)) != cudaSuccess ||
         (e = cudaMallocHost(&b->h_steps[0], step_bytes)) != cudaSuccess ||
         (e = cudaMallocHost(&b->h_steps[1], step_bytes)) != cudaSuccess ||
-        (e = cudaMalloc(&b->d_nitems, sizeof(int))) != cudaSuccess ||
+        (e = cudaMalloc(&b->d_nitems, 2 * sizeof(int))) != cudaSuccess ||
         (e = cudaMalloc(&b->d_part, (592 * kDiagRow + 8) * sizeof(double))) != cudaSuccess ||
         (e = cudaMalloc(&b->d_sites, 2 * 4096 * sizeof(double))) != cudaSuccess ||
         (e = cudaMalloc(&b->d_tmaps, sizeof(CUtensorMap) * 2 * (size_t)max_domains)) != cudaSuccess ||
@@ -360,7 +403,7 @@ int pf_batch_create(int precision, long long budget_bytes, int max_domains, pf_b
         cudaGetLastError();
     }
     cudaMemset(b->d_steps, 0, step_bytes);
-    cudaMemset(b->d_nitems, 0, sizeof(int));
+    cudaMemset(b->d_nitems, 0, 2 * sizeof(int));
     cudaMemset(b->d_status, 0, sizeof(int));
     if (!tmap_encoder()) b->march = 0;   // no tensor-map encoder in this driver: the cp.async passes
     set_grid(b);
@@ -618,6 +661,7 @@ int pf_batch_set_paired(pf_batch* b, int paired)
 {
     if (!b || paired < 0 || paired > 1) return berr(b, PF_E_ARG, "pf_batch_set_paired: 0 or 1");
     b->pair = paired;
+    b->items_dirty = true;
     return PF_OK;
 }
 
@@ -643,6 +687,7 @@ int pf_batch_set_kernel(pf_batch* b, int kernel, int nslot)
     }
     b->march = kernel;
     b->nslot = nslot;
+    b->items_dirty = true;
     return PF_OK;
 }
 
@@ -650,7 +695,8 @@ int pf_batch_set_tile(pf_batch* b, int tile_y, int zchunk)
 {
     if (!b || (tile_y != 4 && tile_y != 8 && tile_y != 16) || zchunk < 1)
         return berr(b, PF_E_ARG, "pf_batch_set_tile: tile_y in {4, 8, 16}, zchunk >= 1");
-    if (tile_y != b->tile_y || zchunk != b->zchunk) {
+    if (b->zauto || tile_y != b->tile_y || zchunk != b->zchunk) {
+        b->zauto = false;
         b->tile_y = tile_y;
         b->zchunk = zchunk;
         b->items_dirty = true;
@@ -674,15 +720,20 @@ int pf_batch_step_async(pf_batch* b, int n_steps)
     long long steps_done = 0;
     int left = n_steps;
     bool launched = false;
+    int n_rows = 0;   // slots in use: only their rows are filled and sent (a table of all slots of a
+                      // 4096-slot batch is 16 MB, 0.3 ms on the link and 2 ms of the host every 8 steps)
+    for (int s = 0; s < (int)b->slots.size(); ++s)
+        if (b->slots[s].used) n_rows = s + 1;
     while (left > 0) {
         const int chunk = std::min(left, kGraphSteps);
         const int hb = b->h_cur;
         BCK(cudaEventSynchronize(b->h_ev[hb]), "step table reuse");
-        const int adv = fill_steps(b, b->h_steps[hb], chunk);
+        const int adv = fill_steps(b, b->h_steps[hb], chunk, n_rows);
         left -= chunk;
         if (adv == 0) break;   // every slot reached its target
-        BCK(cudaMemcpyAsync(b->d_steps, b->h_steps[hb], sizeof(BatchStep) * (size_t)kGraphSteps * b->max_domains,
-                            cudaMemcpyHostToDevice, b->stream),
+        BCK(cudaMemcpy2DAsync(b->d_steps, sizeof(BatchStep) * (size_t)b->max_domains, b->h_steps[hb],
+                              sizeof(BatchStep) * (size_t)n_rows, sizeof(BatchStep) * (size_t)n_rows, kGraphSteps,
+                              cudaMemcpyHostToDevice, b->stream),
             "step table upload");
         BCK(cudaEventRecord(b->h_ev[hb], b->stream), "step table event");
         b->h_cur ^= 1;
@@ -764,7 +815,7 @@ int pf_batch_autotune(pf_batch* b, int steps_per_candidate, int* tile_y, int* zc
     // every candidate runs real steps (results do not depend on the tile
     // shape), one untimed step first
     double best = 1e300;
-    int bty = b->tile_y, bzc = b->zchunk, bpair = 0;
+    int bty = b->tile_y, bzc = b->zchunk, bpair = want_pair(b);
     const bool march = b->march != 0;
     for (int ty : {4, 8, 16})
         for (int zc : {16, 32, 64, 128})

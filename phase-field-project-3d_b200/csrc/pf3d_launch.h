@@ -91,12 +91,13 @@ template <typename S> cudaError_t launch_march_solute(const CUtensorMap& tm, con
                                                       const void* c_in, void* c_out, int zchunk, int* err,
                                                       cudaStream_t st);
 // batch form: tmaps[2 d + b] is the tensor map of buffer b of domain d's
-// phase field; *ctr (zero before the launch) hands out the work items
+// phase field; head = {items, planes per chunk}; *ctr (zero before the launch)
+// hands out the work items
 template <typename S> cudaError_t launch_march_batch(const BatchDomain* doms, const CUtensorMap* tmaps,
                                                      const BatchStep* steps, const BatchItem* items,
-                                                     const int* n_items, int pass, bool one_sweep, bool smooth,
-                                                     int lanes, int nslot, int zchunk, int n_sm, int* ctr,
-                                                     int* err, cudaStream_t st);
+                                                     const int* head, int pass, bool one_sweep, bool smooth,
+                                                     int lanes, int nslot, int n_sm, int* ctr, int* err,
+                                                     cudaStream_t st);
 
 // Solidification tracking of phi: out[3] = {solid fraction, tip position
 // (cells, 1-based), solid cells}; scratch holds nz + 1 words.

@@ -760,7 +760,8 @@ __global__ void __launch_bounds__(32 * TY / L, (FAST ? MarchOcc<S, L, WIN, SOL, 
     }
 }
 
-// many domains: a persistent grid walks the work list.  PASS 0 is the first
+// many domains: a persistent grid walks the work list (head[0] items, chunks
+// of head[1] planes).  PASS 0 is the first
 // pass of a step (temperatura + sweep 1, or the whole step with one sweep),
 // PASS 1 the last (sweep 2 + solute).  tmaps[2 d + b] describes buffer b of
 // domain d's phase field.  Items are handed out dynamically: each CTA starts
@@ -773,7 +774,7 @@ __global__ void __launch_bounds__(32 * TY / L,
                                   (MarchOcc<S, L, WIN, PASS == 1 || ONE_SWEEP, PASS == 0, SMOOTH>::v))
     k_march_batch(const BatchDomain* __restrict__ doms, const CUtensorMap* __restrict__ tmaps,
                   const BatchStep* __restrict__ steps, const BatchItem* __restrict__ items,
-                  const int* __restrict__ n_items, int zchunk, int* __restrict__ ctr, int* __restrict__ err)
+                  const int* __restrict__ head, int* __restrict__ ctr, int* __restrict__ err)
 {
     using V = typename Lanes<S, L>::V;
     constexpr bool SOL = PASS == 1 || ONE_SWEEP;
@@ -786,7 +787,7 @@ __global__ void __launch_bounds__(32 * TY / L,
     unsigned char* smem = align128(smem_raw);
     march_init_barriers<MarchLayout<S, TY, SOL, MarchWin<WIN>::nslot>>(smem);
     uint32_t par = 0;
-    const int n = *n_items;
+    const int n = head[0], zchunk = head[1];
     const int tid = threadIdx.x + 32 * threadIdx.y;
     for (int w = blockIdx.x; w < n;) {
         const BatchItem it = items[w];
@@ -933,8 +934,8 @@ cudaError_t launch_march_last(const CUtensorMap& tm, const DomainDesc& d, const 
 // FP64 runs the reference form, FP32 the fast form; every node's and point's
 // quantities are computed once and shared, where one thread per cell computed
 // six nodes and seven points a cell.  128x128x256 FP64: a whole step of
-// subroutine calls 1146 -> 453 us (a sweep 430 -> 149 us, the solute step with
-// its copy 230 -> 115 us; with the general divisions the sweep took 336 us).
+// subroutine calls 1146 -> 453 us (a sweep 440 -> 149 us, the solute step with
+// its copy 237 -> 115 us; with the general divisions the sweep took 336 us).
 template <typename S>
 cudaError_t launch_march_sweep(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s, const void* c_in,
                                void* phi_out, void* dpp, int zchunk, int* err, cudaStream_t st)
@@ -959,8 +960,8 @@ cudaError_t launch_march_solute(const CUtensorMap& tm, const DomainDesc& d, cons
 // resident on one SM.
 template <typename S, int L, int WIN, int PASS, bool ONE_SWEEP, bool SMOOTH>
 cudaError_t launch_march_batch_t(const BatchDomain* doms, const CUtensorMap* tmaps, const BatchStep* steps,
-                                 const BatchItem* items, const int* n_items, int zchunk, int n_sm, int* ctr,
-                                 int* err, cudaStream_t st)
+                                 const BatchItem* items, const int* head, int n_sm, int* ctr, int* err,
+                                 cudaStream_t st)
 {
     constexpr bool SOL = PASS == 1 || ONE_SWEEP;
     using LY = MarchLayout<S, 8, SOL, MarchWin<WIN>::nslot>;
@@ -974,17 +975,17 @@ cudaError_t launch_march_batch_t(const BatchDomain* doms, const CUtensorMap* tma
         if (e != cudaSuccess) return e;
         per_sm = nb > 0 ? nb : 1;
     }
-    kern<<<n_sm * per_sm, dim3(32, 8 / L), LY::ALLOC, st>>>(doms, tmaps, steps, items, n_items, zchunk, ctr, err);
+    kern<<<n_sm * per_sm, dim3(32, 8 / L), LY::ALLOC, st>>>(doms, tmaps, steps, items, head, ctr, err);
     return cudaGetLastError();
 }
 
 template <typename S>
 cudaError_t launch_march_batch(const BatchDomain* doms, const CUtensorMap* tmaps, const BatchStep* steps,
-                               const BatchItem* items, const int* n_items, int pass, bool one_sweep, bool smooth,
-                               int lanes, int win, int zchunk, int n_sm, int* ctr, int* err, cudaStream_t st)
+                               const BatchItem* items, const int* head, int pass, bool one_sweep, bool smooth,
+                               int lanes, int win, int n_sm, int* ctr, int* err, cudaStream_t st)
 {
 #define PF3D_MB(L, NS, P, ONE, SM) \
-    launch_march_batch_t<S, L, NS, P, ONE, SM>(doms, tmaps, steps, items, n_items, zchunk, n_sm, ctr, err, st)
+    launch_march_batch_t<S, L, NS, P, ONE, SM>(doms, tmaps, steps, items, head, n_sm, ctr, err, st)
 #define PF3D_MW(L, P, ONE, SM) \
     (win == 3 ? PF3D_MB(L, 3, P, ONE, SM) : win == 4 ? PF3D_MB(L, 4, P, ONE, SM) : PF3D_MB(L, 5, P, ONE, SM))
     if (pass == 0) {
