@@ -22,6 +22,7 @@
 #include "pf3d_ckpt.h"
 #include "pf3d_tma.cuh"
 #include "pf3d_tmap.h"
+#include "pf3d_xfer.h"
 
 using namespace pf3d;
 
@@ -193,6 +194,7 @@ int pf_create(const pf_grid* g, const pf_params* p, int precision, pf_ctx** out)
         return set_global_err(PF_E_CUDA, std::string("context set-up: ") + cudaGetErrorString(e));
     }
     ctx->stream = ctx->own_stream;
+    xfer_ref();
     // tensor maps of the phase-field buffers for the TMA plane loads
     ctx->kernel = 1;
     ctx->nslot = 0;
@@ -229,6 +231,7 @@ int pf_destroy(pf_ctx* ctx)
     cudaFreeHost(ctx->h_out);
     cudaStreamDestroy(ctx->own_stream);
     delete ctx;
+    xfer_unref();
     return PF_OK;
 }
 
@@ -344,6 +347,11 @@ int pf_upload(pf_ctx* ctx, int field, const double* host)
 {
     if (!ctx || !host || field < 0 || field > 6) return ctx_err(ctx, PF_E_ARG, "pf_upload: bad argument");
     const pf_grid& g = ctx->g;
+    if (!xfer_pinned(host)) {
+        CK(xfer_to_device(ctx->fld[field], (int)ctx->es, g.nx, ctx->dd.px, (long long)g.ny * g.nz, host, ctx->stream),
+           "pf_upload");
+        return PF_OK;
+    }
     if (is64(ctx)) {
         CK(cudaMemcpy2DAsync(ctx->fld[field], (size_t)ctx->dd.px * 8, host, (size_t)g.nx * 8, (size_t)g.nx * 8,
                              (size_t)g.ny * g.nz, cudaMemcpyHostToDevice, ctx->stream),
@@ -369,6 +377,11 @@ int pf_download(pf_ctx* ctx, int field, double* host)
 {
     if (!ctx || !host || field < 0 || field > 6) return ctx_err(ctx, PF_E_ARG, "pf_download: bad argument");
     const pf_grid& g = ctx->g;
+    if (!xfer_pinned(host)) {
+        CK(xfer_to_host(ctx->fld[field], (int)ctx->es, g.nx, ctx->dd.px, (long long)g.ny * g.nz, host, ctx->stream),
+           "pf_download");
+        return kernel_status(ctx);
+    }
     if (is64(ctx)) {
         CK(cudaMemcpy2DAsync(host, (size_t)g.nx * 8, ctx->fld[field], (size_t)ctx->dd.px * 8, (size_t)g.nx * 8,
                              (size_t)g.ny * g.nz, cudaMemcpyDeviceToHost, ctx->stream),

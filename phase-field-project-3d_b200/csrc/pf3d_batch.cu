@@ -30,6 +30,7 @@
 #include "pf3d_init.cuh"
 #include "pf3d_tma.cuh"
 #include "pf3d_tmap.h"
+#include "pf3d_xfer.h"
 
 using namespace pf3d;
 
@@ -364,6 +365,7 @@ int pf_batch_create(int precision, long long budget_bytes, int max_domains, pf_b
         return set_last_error_global(PF_E_NODEV, "no CUDA device visible");
     }
     pf_batch* b = new pf_batch();
+    xfer_ref();
     b->prec = precision;
     b->es = precision == PF_FP32 ? 4 : 8;
     b->budget = budget_bytes;
@@ -435,6 +437,7 @@ int pf_batch_destroy(pf_batch* b)
         if (ev) cudaEventDestroy(ev);
     if (b->own_stream) cudaStreamDestroy(b->own_stream);
     delete b;
+    xfer_unref();
     return PF_OK;
 }
 
@@ -563,22 +566,14 @@ int pf_batch_upload(pf_batch* b, int slot, int field, const double* host)
     if (!sl || !host || field < 0 || field > 6) return berr(b, PF_E_ARG, "pf_batch_upload: bad argument");
     const pf_grid& g = sl->g;
     void* dst = slot_field(*sl, field);
-    if (b64(b)) {
+    if (b64(b) && xfer_pinned(host)) {
         BCK(cudaMemcpy2DAsync(dst, (size_t)sl->bd.d.px * 8, host, (size_t)g.nx * 8, (size_t)g.nx * 8,
                               (size_t)g.ny * g.nz, cudaMemcpyHostToDevice, b->stream),
             "pf_batch_upload");
-    } else {
-        // through the staging area of the diagnostics buffer is too small; use a temporary
-        const size_t n = (size_t)g.nx * g.ny * g.nz;
-        double* stage = nullptr;
-        BCK(cudaMalloc(&stage, n * sizeof(double)), "pf_batch_upload staging");
-        cudaError_t e = cudaMemcpyAsync(stage, host, n * sizeof(double), cudaMemcpyHostToDevice, b->stream);
-        if (e == cudaSuccess) e = launch_convert_in<float>(sl->bd.d, stage, dst, 0, g.nz, b->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-        cudaFree(stage);
-        if (e != cudaSuccess) return berr(b, PF_E_CUDA, std::string("pf_batch_upload: ") + cudaGetErrorString(e));
+        BCK(cudaStreamSynchronize(b->stream), "pf_batch_upload sync");
+        return PF_OK;
     }
-    BCK(cudaStreamSynchronize(b->stream), "pf_batch_upload sync");
+    BCK(xfer_to_device(dst, (int)b->es, g.nx, sl->bd.d.px, (long long)g.ny * g.nz, host, b->stream), "pf_batch_upload");
     return PF_OK;
 }
 
@@ -588,21 +583,14 @@ int pf_batch_download(pf_batch* b, int slot, int field, double* host)
     if (!sl || !host || field < 0 || field > 6) return berr(b, PF_E_ARG, "pf_batch_download: bad argument");
     const pf_grid& g = sl->g;
     void* src = slot_field(*sl, field);
-    if (b64(b)) {
+    if (b64(b) && xfer_pinned(host)) {
         BCK(cudaMemcpy2DAsync(host, (size_t)g.nx * 8, src, (size_t)sl->bd.d.px * 8, (size_t)g.nx * 8,
                               (size_t)g.ny * g.nz, cudaMemcpyDeviceToHost, b->stream),
             "pf_batch_download");
-    } else {
-        const size_t n = (size_t)g.nx * g.ny * g.nz;
-        double* stage = nullptr;
-        BCK(cudaMalloc(&stage, n * sizeof(double)), "pf_batch_download staging");
-        cudaError_t e = launch_convert_out<float>(sl->bd.d, src, stage, 0, g.nz, b->stream);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(host, stage, n * sizeof(double), cudaMemcpyDeviceToHost, b->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
-        cudaFree(stage);
-        if (e != cudaSuccess) return berr(b, PF_E_CUDA, std::string("pf_batch_download: ") + cudaGetErrorString(e));
+        BCK(cudaStreamSynchronize(b->stream), "pf_batch_download sync");
+        return PF_OK;
     }
-    BCK(cudaStreamSynchronize(b->stream), "pf_batch_download sync");
+    BCK(xfer_to_host(src, (int)b->es, g.nx, sl->bd.d.px, (long long)g.ny * g.nz, host, b->stream), "pf_batch_download");
     return PF_OK;
 }
 

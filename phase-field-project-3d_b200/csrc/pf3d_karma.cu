@@ -10,6 +10,7 @@
 #include "pf3d_hostdesc.h"
 #include "pf3d_karma.cuh"
 #include "pf3d_tmap.h"
+#include "pf3d_xfer.h"
 
 using namespace pf3d;
 
@@ -179,6 +180,7 @@ int pf_karma_create(const pf_karma_params* p, int precision, pf_karma** out)
         return kerr(PF_E_CUDA, std::string("set-up: ") + cudaGetErrorString(e));
     }
     k->stream = k->own_stream;
+    xfer_ref();
     *out = k;
     return PF_OK;
 }
@@ -191,6 +193,7 @@ int pf_karma_destroy(pf_karma* k)
     cudaFreeHost(k->h_tip);
     cudaStreamDestroy(k->own_stream);
     delete k;
+    xfer_unref();
     return PF_OK;
 }
 
@@ -241,17 +244,14 @@ int pf_karma_upload(pf_karma* k, int field, const double* host)
 {
     if (!k || !host || (field != PF_KARMA_PHI && field != PF_KARMA_U)) return kerr(PF_E_ARG, "bad argument");
     const pf_karma_params& p = k->p;
-    const size_t n = (size_t)p.nx * p.ny * p.nz;
-    const void* src = host;
-    std::vector<float> tmp;
-    if (k->prec == PF_FP32) {
-        tmp.resize(n);
-        for (size_t q = 0; q < n; ++q) tmp[q] = (float)host[q];
-        src = tmp.data();
+    cudaError_t e;
+    if (k->prec == PF_FP64 && xfer_pinned(host)) {
+        e = cudaMemcpy2DAsync(karma_field(k, field), (size_t)k->d.px * 8, host, (size_t)p.nx * 8, (size_t)p.nx * 8,
+                              (size_t)p.ny * p.nz, cudaMemcpyHostToDevice, k->stream);
+        if (e == cudaSuccess) e = cudaStreamSynchronize(k->stream);
+    } else {
+        e = xfer_to_device(karma_field(k, field), (int)k->es, p.nx, k->d.px, (long long)p.ny * p.nz, host, k->stream);
     }
-    cudaError_t e = cudaMemcpy2DAsync(karma_field(k, field), (size_t)k->d.px * k->es, src, (size_t)p.nx * k->es,
-                                      (size_t)p.nx * k->es, (size_t)p.ny * p.nz, cudaMemcpyHostToDevice, k->stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(k->stream);
     if (e != cudaSuccess) return kerr(PF_E_CUDA, std::string("upload: ") + cudaGetErrorString(e));
     return PF_OK;
 }
@@ -260,21 +260,14 @@ int pf_karma_download(pf_karma* k, int field, double* host)
 {
     if (!k || !host || field < PF_KARMA_PHI || field > PF_KARMA_DPHI) return kerr(PF_E_ARG, "bad argument");
     const pf_karma_params& p = k->p;
-    const size_t n = (size_t)p.nx * p.ny * p.nz;
-    std::vector<float> tmp;
-    void* dst = host;
-    if (k->prec == PF_FP32) {
-        tmp.resize(n);
-        dst = tmp.data();
-    }
-    cudaError_t e = cudaMemcpy2DAsync(dst, (size_t)p.nx * k->es, karma_field(k, field), (size_t)k->d.px * k->es,
-                                      (size_t)p.nx * k->es, (size_t)p.ny * p.nz, cudaMemcpyDeviceToHost, k->stream);
+    cudaError_t e;
+    if (k->prec == PF_FP64 && xfer_pinned(host))
+        e = cudaMemcpy2DAsync(host, (size_t)p.nx * 8, karma_field(k, field), (size_t)k->d.px * 8, (size_t)p.nx * 8,
+                              (size_t)p.ny * p.nz, cudaMemcpyDeviceToHost, k->stream);
+    else
+        e = xfer_to_host(karma_field(k, field), (int)k->es, p.nx, k->d.px, (long long)p.ny * p.nz, host, k->stream);
     if (e != cudaSuccess) return kerr(PF_E_CUDA, std::string("download: ") + cudaGetErrorString(e));
-    const int rc = karma_wait(k, "download");
-    if (rc != PF_OK) return rc;
-    if (k->prec == PF_FP32)
-        for (size_t q = 0; q < n; ++q) host[q] = (double)tmp[q];
-    return PF_OK;
+    return karma_wait(k, "download");
 }
 
 int pf_karma_seed(pf_karma* k)
