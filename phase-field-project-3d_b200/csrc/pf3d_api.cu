@@ -77,7 +77,7 @@ struct pf_ctx {
     int zfill[3];            // ... cached by the CTAs an SM holds (index: kMarchOcc)
     int n_sm;
     int kernel;              // PF_OPT_KERNEL: 1 TMA-staged march passes, 0 the cp.async passes
-    int nslot;               // PF_OPT_NSLOT: window mode of the march passes (0: 3)
+    int nslot;               // PF_OPT_NSLOT: accepted and reported, all modes run the 3-plane windows
     CUtensorMap tmap[2];     // tensor maps of the two phase-field buffers (32 x 8 march tiles)
     void* tmap_buf[2];       // their base addresses
     int* d_status;           // kernel status word: 0, or the code a kernel left there
@@ -698,15 +698,14 @@ static int one_step(pf_ctx* ctx)
         // TMA-staged passes: two cells per thread unless PF_OPT_PAIRED says
         // otherwise (default: FP32 only) or the deck draws the smooth noise
         const int lanes = ((ctx->paired == 2 || (ctx->paired == 1 && !is64(ctx))) && p.ruido_tipo != 2) ? 2 : 1;
-        const int nslot = ctx->nslot ? ctx->nslot : 3;
         const int occ_q = (is64(ctx) && p.ruido_tipo == 2) ? 0 : (lanes == 2 && !is64(ctx)) ? 2 : 1;
         const int zchunk = ctx->zchunk_set ? ctx->zchunk : ctx->zfill[occ_q];
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         f.phi_mid = B;
         if (ctx->ktiming) { e0 = new_event(); e1 = new_event(); cudaEventRecord(e0, ctx->stream); }
-        CK(is64(ctx) ? launch_march_first<double>(tm_of(ctx, A), ctx->dd, s, f, nsw == 1, lanes, nslot, zchunk,
+        CK(is64(ctx) ? launch_march_first<double>(tm_of(ctx, A), ctx->dd, s, f, nsw == 1, lanes, zchunk,
                                                   ctx->d_status, ctx->stream)
-                     : launch_march_first<float>(tm_of(ctx, A), ctx->dd, s, f, nsw == 1, lanes, nslot, zchunk,
+                     : launch_march_first<float>(tm_of(ctx, A), ctx->dd, s, f, nsw == 1, lanes, zchunk,
                                                  ctx->d_status, ctx->stream),
            nsw == 1 ? "march step (single sweep)" : "march heat + sweep 1");
         if (ctx->ktiming) { cudaEventRecord(e1, ctx->stream); ctx->ev_first.push_back({e0, e1}); }
@@ -725,9 +724,9 @@ static int one_step(pf_ctx* ctx)
             f2.phi_mid = cur;
             f2.phi_new = oth;
             if (ctx->ktiming) { e0 = new_event(); e1 = new_event(); cudaEventRecord(e0, ctx->stream); }
-            CK(is64(ctx) ? launch_march_last<double>(tm_of(ctx, cur), ctx->dd, s, f2, lanes, nslot, zchunk,
+            CK(is64(ctx) ? launch_march_last<double>(tm_of(ctx, cur), ctx->dd, s, f2, lanes, zchunk,
                                                      ctx->d_status, ctx->stream)
-                         : launch_march_last<float>(tm_of(ctx, cur), ctx->dd, s, f2, lanes, nslot, zchunk,
+                         : launch_march_last<float>(tm_of(ctx, cur), ctx->dd, s, f2, lanes, zchunk,
                                                     ctx->d_status, ctx->stream),
                "march last sweep + solute");
             if (ctx->ktiming) { cudaEventRecord(e1, ctx->stream); ctx->ev_last.push_back({e0, e1}); }

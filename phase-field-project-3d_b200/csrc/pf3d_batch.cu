@@ -87,13 +87,13 @@ struct pf_batch {
     int zc = 64;                       // chunk of the current work list
     int pair = -1;                     // 32 x 8 tiles with two cells per thread; -1: FP32 yes, FP64 no
     int march = 1;                     // TMA-staged march passes (32 x 8 tiles); 0: the cp.async passes
-    int nslot = 0;                     // window mode of the march passes (0: 3)
+    int nslot = 0;                     // window mode as set (all run the 3-plane windows)
     CUtensorMap* d_tmaps = nullptr;    // 2 per slot: the tensor maps of its phase-field buffers
     int* d_ctr = nullptr;              // work-item counters of a graph's launches (2 per step)
     int* d_status = nullptr;           // kernel status word (0, or the code a kernel left there)
     cudaStream_t own_stream = nullptr, stream = nullptr;
     cudaGraphExec_t graph = nullptr;
-    int graph_ty = 0, graph_zc = 0, graph_nsm = 0, graph_nsw = 0, graph_march = -1, graph_nslot = 0;
+    int graph_ty = 0, graph_zc = 0, graph_nsm = 0, graph_nsw = 0, graph_march = -1;
     bool graph_smooth = false, graph_pair = false;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
     double last_ms = 0.0;
@@ -217,7 +217,6 @@ static int capture_graph(pf_batch* b)
 {
     const bool smooth = any_smooth(b);
     const bool march = use_march(b);
-    const int nslot = b->nslot ? b->nslot : 3;
     // two cells per thread on 32 x 8 tiles: the march passes in either
     // precision (not with the smooth noise); the cp.async passes where it was
     // asked for, in FP32 only, on decks without heat diffusion (their boundary
@@ -227,7 +226,7 @@ static int capture_graph(pf_batch* b)
     const int zc = march ? 0 : b->zchunk;   // the march passes read their chunk from the work list's head
     if (b->graph && b->graph_ty == b->tile_y && b->graph_zc == zc && b->graph_nsm == b->n_sm &&
         b->graph_nsw == b->nsw && b->graph_smooth == smooth && b->graph_pair == pair &&
-        b->graph_march == (int)march && b->graph_nslot == nslot)
+        b->graph_march == (int)march)
         return PF_OK;
     if (b->graph) {
         cudaGraphExecDestroy(b->graph);
@@ -247,10 +246,10 @@ static int capture_graph(pf_batch* b)
                 const int lanes = pair ? 2 : 1;
                 for (int pass = 0; pass <= (one ? 0 : 1) && e == cudaSuccess; ++pass)
                     e = b64(b) ? launch_march_batch<double>(b->d_doms, b->d_tmaps, st, b->d_items, b->d_nitems, pass,
-                                                            one, smooth && pass == 0, lanes, nslot, b->n_sm,
+                                                            one, smooth && pass == 0, lanes, b->n_sm,
                                                             b->d_ctr + 2 * k + pass, b->d_status, cs)
                                : launch_march_batch<float>(b->d_doms, b->d_tmaps, st, b->d_items, b->d_nitems, pass,
-                                                           one, smooth && pass == 0, lanes, nslot, b->n_sm,
+                                                           one, smooth && pass == 0, lanes, b->n_sm,
                                                            b->d_ctr + 2 * k + pass, b->d_status, cs);
                 continue;
             }
@@ -286,7 +285,6 @@ static int capture_graph(pf_batch* b)
     b->graph_smooth = smooth;
     b->graph_pair = pair;
     b->graph_march = (int)march;
-    b->graph_nslot = nslot;
     return PF_OK;
 }
 

@@ -73,14 +73,13 @@ template <typename T> cudaError_t launch_fused_batch_pair(const BatchDomain* dom
                                                           bool one_sweep, int zchunk, int n_sm, cudaStream_t st);
 
 // TMA-staged z-marching passes (pf3d_march.cuh): 32 x 8 tiles, the input
-// phase field through the tensor map `tm`, `lanes` cells per thread (1 or 2),
-// `nslot` node-window planes (3 or 4); a plane load that does not arrive sets
-// *err.  Same outputs, bit for bit, as launch_fused_first / _last.
+// phase field through the tensor map `tm`, `lanes` cells per thread (1 or 2);
+// a plane load that does not arrive sets *err.  Same outputs, bit for bit, as launch_fused_first / _last.
 template <typename S> cudaError_t launch_march_first(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s,
-                                                     const Fields& f, bool with_solute, int lanes, int nslot,
-                                                     int zchunk, int* err, cudaStream_t st);
+                                                     const Fields& f, bool with_solute, int lanes, int zchunk,
+                                                     int* err, cudaStream_t st);
 template <typename S> cudaError_t launch_march_last(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s,
-                                                    const Fields& f, int lanes, int nslot, int zchunk, int* err,
+                                                    const Fields& f, int lanes, int zchunk, int* err,
                                                     cudaStream_t st);
 // one subroutine alone (FP64: reference form): a phase sweep (dpp may be null)
 // and the solute update
@@ -96,7 +95,7 @@ template <typename S> cudaError_t launch_march_solute(const CUtensorMap& tm, con
 template <typename S> cudaError_t launch_march_batch(const BatchDomain* doms, const CUtensorMap* tmaps,
                                                      const BatchStep* steps, const BatchItem* items,
                                                      const int* head, int pass, bool one_sweep, bool smooth,
-                                                     int lanes, int nslot, int n_sm, int* ctr, int* err,
+                                                     int lanes, int n_sm, int* ctr, int* err,
                                                      cudaStream_t st);
 
 // Solidification tracking of phi: out[3] = {solid fraction, tip position

@@ -13,9 +13,8 @@
 //    the context's status word and the CTA stops (pf3d_tma.cuh).
 //  * Node windows.  The anisotropy quantities (eps^2, exy, eyz, ezx) of every
 //    node of the tile and its 1-cell ring, and the solute point quantities
-//    (Gamma bracket, mu), are computed once per plane into 3- or 4-plane
-//    windows; the window mode (MarchWin) says how many and how many barriers
-//    a plane takes, and whether the own column's values roll in registers.
+//    (Gamma bracket, mu), are computed once per plane into 3-plane windows,
+//    one barrier a plane (MarchLayout).
 //  * Uniform arithmetic, fan-out stores.  Every cell of every tile -- also
 //    the tiles on the domain boundary -- goes through the same arithmetic
 //    (two cells per thread as lane pairs when L = 2, packed f32x2 in FP32).
@@ -52,56 +51,51 @@ template <typename S> struct Lanes<S, 2> {
     static __device__ __forceinline__ S get(const V& v, int l) { return l ? v.y() : v.x(); }
 };
 
-// Window modes of the march passes (one barrier per plane in each):
-//   3: node / solute-point windows of 3 planes.  The cells of plane z read
-//      plane z's nodes and points at their neighbours' positions, written
-//      by other threads before the previous plane's barrier, and those of
-//      planes z-1 and z+1 only at their own position, written by the same
-//      thread; so when the nodes of plane z+1 overwrite plane z-2's slot,
-//      the last cross-thread reader of that slot (the cells of plane z-2)
-//      is behind the previous plane's barrier, and no second barrier is
-//      needed;
-//   4: windows of 4 planes (a spare slot, same results);
-//   5: the own column's values rolled in registers along z -- the phase
-//      values of planes z-1, z, z+1 at the cell and its four axis
-//      neighbours, the cell's node quantities of planes z-1, z, z+1 and its
-//      solute-point quantities of the same planes -- so the stencil reads
-//      from shared memory only the in-plane neighbours of plane z (the
-//      diagonal phase values and the four neighbour nodes and points),
-//      with windows of 3 planes.
-template <int WIN> struct MarchWin {
-    static_assert(WIN == 3 || WIN == 4 || WIN == 5, "window mode 3, 4 or 5");
-    static constexpr int nslot = (WIN == 4) ? 4 : 3;
-    static constexpr bool roll = WIN == 5;
-};
-
-// Shared-memory layout of one tile (bytes from a 128-byte aligned base).
-template <typename S, int TY, bool SOL, int NSLOT, bool PHASE = true, bool FAST = true>
+// Shared-memory layout of one tile (bytes from a 128-byte aligned base): six
+// phase planes (z-1 .. z+4), their barriers, and the node / solute-point
+// windows of three planes, a plane's node and point arrays in one slot.
+//
+// Three planes suffice with one barrier a plane: the cells of plane z read
+// plane z's nodes and points at their neighbours' positions, written by other
+// threads before the previous plane's barrier, and those of planes z-1 and
+// z+1 only at their own position, written by the same thread; so when the
+// nodes of plane z+1 overwrite plane z-2's slot, the last cross-thread reader
+// of that slot (the cells of plane z-2) is behind the previous plane's
+// barrier.
+template <typename S, int TY, bool SOL, bool PHASE = true, bool FAST = true>
 struct MarchLayout {
     static constexpr int TX = 32;
+    static constexpr int ES = (int)sizeof(S);
     // the TMA box starts XOFF cells left of the tile: x * sizeof(S) must be a
     // multiple of 16 bytes (tile origins are multiples of 32 cells)
     static constexpr int XOFF = (sizeof(S) == 8) ? 2 : 4;
     static constexpr int TW = TX + 2 * XOFF;       // phase tile width (box x)
     static constexpr int PH = TY + 4;              // phase tile height (box y)
     static constexpr int NW = TX + 2, NH = TY + 2; // node / point tile (ring 1)
-    static constexpr int NQ = NW * NH;
-    static constexpr int NPHI = 6;                 // phase planes z-1 .. z+4
-    static constexpr int PHI_SLOT = TW * PH;       // elements per phase slot
-    static constexpr int PHI_BYTES = PHI_SLOT * (int)sizeof(S);
+    static constexpr int NB = NW * NH * ES;        // bytes of one node or point array
+    static constexpr int NPHI = 6;
+    static constexpr int PHI_BYTES = TW * PH * ES;
     static_assert(PHI_BYTES % 128 == 0, "TMA destinations are 128-byte aligned");
     static constexpr int BAR_OFF = NPHI * PHI_BYTES;
     static constexpr int NODE_OFF = (BAR_OFF + NPHI * 8 + 127) / 128 * 128;
-    static constexpr int NODE_SLOT = 4 * NQ;       // eps^2, exy, eyz, ezx
-    static constexpr int SOL_OFF = NODE_OFF + (PHASE ? NSLOT * NODE_SLOT * (int)sizeof(S) : 0);
-    static constexpr int SOL_SLOT = (FAST ? 2 : 3) * NQ;   // Gamma bracket, mu; reference form 1/GAMMA twice, mu
-    static constexpr int BYTES = SOL_OFF + (SOL ? NSLOT * SOL_SLOT * (int)sizeof(S) : 0);
+    // arrays of a slot: eps^2, exy, eyz, ezx; Gamma bracket, mu (reference
+    // form 1/GAMMA, mu, 1/GAMMA of the solid)
+    static constexpr int Q_SOL = PHASE ? 4 : 0;
+    static constexpr int SLOT = (Q_SOL + (SOL ? (FAST ? 2 : 3) : 0)) * NB;
+    static constexpr int BYTES = NODE_OFF + 3 * SLOT;
     static constexpr int ALLOC = BYTES + 128;      // slack to align the dynamic base
 };
 
+// shared memory by 32-bit address (base + an offset the compiler folds into
+// the instruction)
+__device__ __forceinline__ void lds(uint32_t a, double& v) { asm volatile("ld.shared.f64 %0, [%1];" : "=d"(v) : "r"(a)); }
+__device__ __forceinline__ void lds(uint32_t a, float& v) { asm volatile("ld.shared.f32 %0, [%1];" : "=f"(v) : "r"(a)); }
+__device__ __forceinline__ void sts(uint32_t a, double v) { asm volatile("st.shared.f64 [%0], %1;" ::"r"(a), "d"(v)); }
+__device__ __forceinline__ void sts(uint32_t a, float v) { asm volatile("st.shared.f32 [%0], %1;" ::"r"(a), "f"(v)); }
+
 // temperatura at one own cell (temp_body.inc:31-41): the neighbours of TOLD
 // are read only when the deck has heat diffusion (D != 0)
-template <typename S>
+template <typename S, int HQ>
 __device__ __forceinline__ S heat_at(const S* __restrict__ T_old, long long id, long long px, long long pl, S PP,
                                      S dppv, const KC<S>& c)
 {
@@ -110,15 +104,7 @@ __device__ __forceinline__ S heat_at(const S* __restrict__ T_old, long long id, 
         TE = T_old[id + 1]; TW = T_old[id - 1]; TN = T_old[id + px]; TS = T_old[id - px];
         TT = T_old[id + pl]; TB = T_old[id - pl];
     }
-    return heat_new<S>(PP, dppv, TE, TW, TN, TS, TT, TB, c);
-}
-
-// (a + k) mod N for a in [0, N) and k in [0, N)
-template <int N>
-__device__ __forceinline__ int wrap_add(int a, int k)
-{
-    const int t = a + k;
-    return t >= N ? t - N : t;
+    return heat_new<S, true, HQ>(PP, dppv, TE, TW, TN, TS, TT, TB, c);
 }
 
 // the dynamic shared-memory base rounded up to 128 bytes.  The offset is
@@ -149,12 +135,29 @@ __device__ __forceinline__ void march_init_barriers(unsigned char* smem)
 // parity of each plane barrier across the tiles a CTA processes (every load
 // issued is waited for).  Returns false if a plane load did not arrive in
 // time; the CTA must then stop.  SPLIT: a second copy of the plane body for
-// the interior planes, without their z checks (single domains; a batch's
-// short items gain less than the larger code costs them, measured).  PHASE =
-// false leaves the phase sweep out (the solute subroutine alone); FAST = false
-// is the reference form of the per-subroutine entry points (FP64, one lane).
-template <typename S, int L, int TY, int WIN, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool SPLIT = true,
-          bool PHASE = true, bool FAST = true>
+// the interior planes, without their z checks (FP64 single domains).  INT: every
+// column and row of the tile lies in [3, N-4], so no cell needs a check or a
+// second store (FP64).
+// PHASE = false leaves the phase sweep out (the solute subroutine alone);
+// FAST = false is the reference form of the per-subroutine entry points (FP64,
+// one lane).
+//
+// The arithmetic is a third to a half of what a plane executes: the rest is
+// addresses, conditions and moves, and every thread repeats it in every
+// plane.  So shared memory is reached by 32-bit addresses kept per plane of
+// the windows and rotated with them (all neighbours are immediate offsets,
+// ring items one added delta), global memory by a plane pointer that is the
+// same for the CTA plus a 32-bit offset, and the conditions that only tiles on
+// the domain's faces need exist in their copy of the body alone.  FP64
+// 340x340x200, pass 1 / pass 2: 602 + 815 -> 553 + 744 us (563 / 758 -> 490 /
+// 685 instructions a cell on 256x256x128); FP32 256^3: 292 + 351 -> 262 + 305
+// us.  Also tried: one loop over own cells and ring items (half the node and
+// point code; 2 % slower for the run-time addresses), the prologue as two
+// planes of the march without cells (small domains 3 to 18 % slower for the
+// barriers), the logarithm's coefficients in the constant bank (pass 2 10 %
+// slower), 2 CTAs an SM with 128 registers (4 % slower).
+template <typename S, int L, int TY, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool SPLIT, bool PHASE, bool FAST,
+          int HQ, bool INT>
 __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, const KC<typename Lanes<S, L>::V>& cv,
                                            const CUtensorMap* tm, const S* __restrict__ c_in,
                                            S* __restrict__ phi_out, S* __restrict__ dpp, S* __restrict__ c_out,
@@ -163,20 +166,19 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
 {
     using LN = Lanes<S, L>;
     using V = typename LN::V;
-    constexpr int NSLOT = MarchWin<WIN>::nslot;
-    constexpr bool ROLL = MarchWin<WIN>::roll;
-    using LY = MarchLayout<S, TY, SOL, NSLOT, PHASE, FAST>;
-    constexpr int TX = 32, TW = LY::TW, NW = LY::NW, NH = LY::NH, NQ = LY::NQ, XOFF = LY::XOFF;
-    constexpr int TR = TY / L;                                    // thread rows; lane l owns row ty + l*TR
+    using LY = MarchLayout<S, TY, SOL, PHASE, FAST>;
+    constexpr int ES = LY::ES, TX = 32, NW = LY::NW, NH = LY::NH, NB = LY::NB, XOFF = LY::XOFF;
+    constexpr int TR = TY / L;                                   // thread rows; lane l owns row ty + l*TR
+    constexpr int PR = LY::TW * ES, NR = NW * ES;                // bytes of a phase / node row
+    constexpr int LP = TR * PR, LNB = TR * NR;                   // from a thread's lane to its next
     constexpr int ran_mode = (HEAT && !DPPW) ? 1 : ((!HEAT && DPPW && SOL) ? 2 : 0);
     constexpr int NRING = (L == 1) ? 2 * NW + 2 * TY : NW + TY;  // ring items (pairs when L = 2)
+    constexpr int NT = 32 * TY / L;
     static_assert(TY % L == 0, "tile height must be a multiple of the lanes");
+    static_assert(2 * NRING <= NT, "the node and solute ring threads are disjoint");
 
-    S* const sphi = reinterpret_cast<S*>(smem);
-    const uint32_t bar0 = smem_u32(smem + LY::BAR_OFF);
-    S* const snode = reinterpret_cast<S*>(smem + LY::NODE_OFF);
-    S* const ssol = reinterpret_cast<S*>(smem + LY::SOL_OFF);
-
+    const uint32_t sb = smem_u32(smem);
+    const uint32_t bar0 = sb + LY::BAR_OFF;
     const int nx = d.nx, ny = d.ny, nz = d.nz;
     const long long px = d.px, pl = d.plane;
     const int x0 = bx * TX, y0 = by * TY;
@@ -186,51 +188,46 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
     const int tx = threadIdx.x, ty = threadIdx.y;
     const int tid = tx + TX * ty;
     const bool lead = tid == 0;
-    const int x = x0 + tx;
+    const bool tile_int = INT || (x0 >= 3 && x0 + TX + 3 <= nx && y0 >= 3 && y0 + TY + 3 <= ny);
 
-    // ---- the cells of this thread (lanes) ----
-    int yv[L];
-    bool own[L];
-    long long col[L];
-    int phi_off[L], node_off[L];
-#pragma unroll
-    for (int l = 0; l < L; ++l) {
-        yv[l] = y0 + ty + l * TR;
-        own[l] = x < nx && yv[l] < ny;
-        col[l] = (long long)x + (long long)yv[l] * px;
-        phi_off[l] = (ty + l * TR + 2) * TW + (tx + XOFF);
-        node_off[l] = (ty + l * TR + 1) * NW + (tx + 1);
-    }
-    // ---- the ring items of this thread: node-tile positions.  The first
-    // NRING threads compute the ring's node quantities, the last NRING its
-    // solute points (solute passes), so that no warp carries both ring parts
-    // of a plane while the others wait for it at the plane's barrier ----
-    constexpr int NT = 32 * TY / L;
-    static_assert(2 * NRING <= NT, "the node and solute ring threads are disjoint");
-    int rlx[L], rly[L];
+    // ---- the cells of this thread, and its ring items.  The first NRING
+    // threads compute the ring's node quantities, the last NRING its solute
+    // points (solute passes), so that no warp carries both ring parts of a
+    // plane while the others wait for it at the plane's barrier ----
+    const uint32_t own_phi = (uint32_t)((ty + 2) * PR + (tx + XOFF) * ES);   // lane 0, in a phase slot
+    const uint32_t own_node = (uint32_t)((ty + 1) * NR + (tx + 1) * ES);     // lane 0, in a node array
     const bool ring = tid < NRING;                      // ring nodes
     const bool ring_s = SOL && tid >= NT - NRING;       // ring solute points
-    if (L == 1) {
-        int r = ring ? tid : (ring_s ? tid - (NT - NRING) : 0);
-        if (r < NW) { rlx[0] = r; rly[0] = 0; }
-        else if ((r -= NW) < NW) { rlx[0] = r; rly[0] = NH - 1; }
-        else if ((r -= NW) < TY) { rlx[0] = 0; rly[0] = 1 + r; }
-        else { r -= TY; rlx[0] = NW - 1; rly[0] = 1 + r; }
-    } else {
-        const int r = ring ? tid : (ring_s ? tid - (NT - NRING) : 0);
-        if (r < NW) { rlx[0] = r; rly[0] = 0; rlx[L - 1] = r; rly[L - 1] = NH - 1; }
-        else { rlx[0] = 0; rly[0] = 1 + (r - NW); rlx[L - 1] = NW - 1; rly[L - 1] = 1 + (r - NW); }
-    }
-    bool rin[L];
-    long long rcol[L];
-    int rphi_off[L], rnode_off[L];
+    uint32_t col[L], rcol[L];      // element offsets in the plane: own cells, ring points
+    uint32_t rphi[L], rnode[L];    // bytes from the thread's own position (lane 0) to its ring items
+    bool own[L], xyin[L], rin[L];
+    {
+        int r = ring ? tid : (ring_s ? tid - (NT - NRING) : 0), rx[L], ry[L];
+        if (L == 1) {
+            if (r < NW) { rx[0] = r; ry[0] = 0; }
+            else if ((r -= NW) < NW) { rx[0] = r; ry[0] = NH - 1; }
+            else if ((r -= NW) < TY) { rx[0] = 0; ry[0] = 1 + r; }
+            else { r -= TY; rx[0] = NW - 1; ry[0] = 1 + r; }
+        } else if (r < NW) {
+            rx[0] = rx[L - 1] = r;
+            ry[0] = 0;
+            ry[L - 1] = NH - 1;
+        } else {
+            rx[0] = 0;
+            rx[L - 1] = NW - 1;
+            ry[0] = ry[L - 1] = 1 + (r - NW);
+        }
 #pragma unroll
-    for (int l = 0; l < L; ++l) {
-        const int gx = x0 - 1 + rlx[l], gy = y0 - 1 + rly[l];
-        rin[l] = ring_s && gx >= 0 && gx < nx && gy >= 0 && gy < ny;   // a ring point's concentration is read
-        rcol[l] = (long long)gx + (long long)gy * px;
-        rphi_off[l] = (rly[l] + 1) * TW + (rlx[l] - 1 + XOFF);
-        rnode_off[l] = rly[l] * NW + rlx[l];
+        for (int l = 0; l < L; ++l) {
+            const int x = x0 + tx, y = y0 + ty + l * TR, gx = x0 - 1 + rx[l], gy = y0 - 1 + ry[l];
+            own[l] = INT || (x < nx && y < ny);
+            xyin[l] = INT || (x >= 1 && x <= nx - 2 && y >= 1 && y <= ny - 2);
+            rin[l] = ring_s && (INT || (gx >= 0 && gx < nx && gy >= 0 && gy < ny));   // its concentration is read
+            col[l] = (uint32_t)x + (uint32_t)y * (uint32_t)px;
+            rcol[l] = (uint32_t)gx + (uint32_t)gy * (uint32_t)px;
+            rphi[l] = (uint32_t)((ry[l] + 1) * PR + (rx[l] - 1 + XOFF) * ES) - own_phi;
+            rnode[l] = (uint32_t)(ry[l] * NR + rx[l] * ES) - own_node;
+        }
     }
 
     // ---- plane loads ----
@@ -238,7 +235,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
     auto issue = [&](int p, int s) {   // one thread: plane p into its slot s = p mod 6
         const uint32_t bar = bar0 + 8 * s;
         mbar_arrive_expect_tx(bar, (uint32_t)LY::PHI_BYTES);
-        tma_load_3d(smem_u32(sphi + s * LY::PHI_SLOT), tm, x0 - XOFF, y0 - 2, p, bar);
+        tma_load_3d(sb + s * LY::PHI_BYTES, tm, x0 - XOFF, y0 - 2, p, bar);
         pend |= 1u << s;
     };
     auto wait_plane = [&](int s) -> bool {   // the load into slot s has landed
@@ -257,180 +254,122 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
         for (int s = 0; s < 6; ++s)
             if ((pend >> s) & 1u) mbar_wait(bar0 + 8 * s, (par >> s) & 1u);
     };
+    auto phi_at = [&](int s) { return sb + (uint32_t)(s * LY::PHI_BYTES) + own_phi; };        // own cell, slot s
+    auto node_at = [&](int s) { return sb + (uint32_t)(LY::NODE_OFF + s * LY::SLOT) + own_node; };
 
-    // the node quantities of one set of items from their gradient; stored
-    // into the slot `dst`; the own items' eps^2, eyz, ezx also into `keep`
-    auto node_store = [&](S* dst, const int* off_node, V gx, V gy, V gz, S (*keep)[3]) {
+    // own lanes (ring = false) or ring items of a plane: the address of lane l
+    auto pa = [&](uint32_t a, int l, bool rg) { return rg ? a + rphi[l] : a + (uint32_t)(l * LP); };
+    auto na = [&](uint32_t a, int l, bool rg) { return rg ? a + rnode[l] : a + (uint32_t)(l * LNB); };
+    // the difference of two neighbours, lane by lane
+    auto ldv = [&](uint32_t a, int off, bool rg) -> V {
+        S t[L];
+#pragma unroll
+        for (int l = 0; l < L; ++l) lds(pa(a, l, rg) + (uint32_t)off, t[l]);
+        return LN::make(t);
+    };
+    auto ldn = [&](uint32_t a, int off) -> V {   // own lanes' neighbour in a node / point array
+        S t[L];
+#pragma unroll
+        for (int l = 0; l < L; ++l) lds(a + (uint32_t)(l * LNB + off), t[l]);
+        return LN::make(t);
+    };
+    auto stn = [&](uint32_t a, int q, V v, bool rg) {
+#pragma unroll
+        for (int l = 0; l < L; ++l) sts(na(a, l, rg) + (uint32_t)(q * NB), LN::get(v, l));
+    };
+    // node quantities of a plane into its slot `dst`, from the phase planes
+    // below, at and above it (own addresses)
+    auto node_one = [&](uint32_t dst, uint32_t m, uint32_t p0, uint32_t pp, bool rg) {
+        const V gx = grad<V, FAST>(ldv(p0, ES, rg), ldv(p0, -ES, rg), cv.dx, cv.hx);
+        const V gy = grad<V, FAST>(ldv(p0, PR, rg), ldv(p0, -PR, rg), cv.dy, cv.hy);
+        const V gz = grad<V, FAST>(ldv(pp, 0, rg), ldv(m, 0, rg), cv.dz, cv.hz);
         const Node<V> q = aniso_node<V, FAST>(gx, gy, gz, cv);
-        const V eps2 = q.eps * q.eps;   // the stencil reads eps only squared
-#pragma unroll
-        for (int l = 0; l < L; ++l) {
-            S* o = dst + off_node[l];
-            o[0] = LN::get(eps2, l);
-            o[NQ] = LN::get(q.exy, l);
-            o[2 * NQ] = LN::get(q.eyz, l);
-            o[3 * NQ] = LN::get(q.ezx, l);
-            if (keep) {
-                keep[l][0] = LN::get(eps2, l);
-                keep[l][1] = LN::get(q.eyz, l);
-                keep[l][2] = LN::get(q.ezx, l);
-            }
-        }
+        stn(dst, 0, q.eps * q.eps, rg);   // the stencil reads eps only squared
+        stn(dst, 1, q.exy, rg);
+        stn(dst, 2, q.eyz, rg);
+        stn(dst, 3, q.ezx, rg);
     };
-    // node quantities of plane n into its slot, from phase planes n-1, n, n+1
-    // in shared memory (own items' values also into `keep` when given)
-    auto node_plane = [&](int sl, const S* pm, const S* p0, const S* pp, S (*keep)[3]) {
-        S* dst = snode + sl * LY::NODE_SLOT;
-        auto one = [&](const int* off_phi, const int* off_node, S (*kp)[3]) {
-            S a[L], b[L];
-#pragma unroll
-            for (int l = 0; l < L; ++l) { a[l] = p0[off_phi[l] + 1]; b[l] = p0[off_phi[l] - 1]; }
-            const V gx = grad<V, FAST>(LN::make(a), LN::make(b), cv.dx, cv.hx);
-#pragma unroll
-            for (int l = 0; l < L; ++l) { a[l] = p0[off_phi[l] + TW]; b[l] = p0[off_phi[l] - TW]; }
-            const V gy = grad<V, FAST>(LN::make(a), LN::make(b), cv.dy, cv.hy);
-#pragma unroll
-            for (int l = 0; l < L; ++l) { a[l] = pp[off_phi[l]]; b[l] = pm[off_phi[l]]; }
-            const V gz = grad<V, FAST>(LN::make(a), LN::make(b), cv.dz, cv.hz);
-            node_store(dst, off_node, gx, gy, gz, kp);
-        };
-        one(phi_off, node_off, keep);
-        if (ring) one(rphi_off, rnode_off, nullptr);
+    auto node_plane = [&](uint32_t dst, uint32_t m, uint32_t p0, uint32_t pp) {
+        node_one(dst, m, p0, pp, false);
+        if (ring) node_one(dst, m, p0, pp, true);
     };
-    // solute point quantities of plane s into its slot, from phase plane s
-    // and the concentration of that plane at the own (co) and ring (cr)
-    // points; the own points' values also into `keep` when given, and their
-    // phase values taken from `ownp` when given
-    auto sol_plane = [&](int sl, const S* p0, const S* co, const S* cr, S (*keep)[2], const S* ownp) {
-        S* dst = ssol + sl * LY::SOL_SLOT;
-        auto one = [&](const int* off_phi, const int* off_node, const S* cc, S (*kp)[2], const S* op) {
-            S a[L];
-#pragma unroll
-            for (int l = 0; l < L; ++l) a[l] = op ? op[l] : p0[off_phi[l]];
-            const SolNode<V> q = sol_node<V, FAST>(LN::make(a), LN::make(cc), cv);
-#pragma unroll
-            for (int l = 0; l < L; ++l) {
-                S* o = dst + off_node[l];
-                o[0] = LN::get(FAST ? q.br : q.il, l);
-                o[NQ] = LN::get(q.mu, l);
-                if (!FAST) o[2 * NQ] = LN::get(q.is, l);
-                if (kp) {
-                    kp[l][0] = LN::get(q.br, l);
-                    kp[l][1] = LN::get(q.mu, l);
-                }
-            }
-        };
-        one(phi_off, node_off, co, keep, ownp);
-        if (ring_s) one(rphi_off, rnode_off, cr, nullptr, nullptr);
+    // solute point quantities of a plane into its slot, from its phase plane
+    // and the concentration at the own (co) and ring (cr) points
+    auto sol_one = [&](uint32_t dst, uint32_t p0, const S* cc, bool rg) {
+        const SolNode<V> q = sol_node<V, FAST, HQ>(ldv(p0, 0, rg), LN::make(cc), cv);
+        stn(dst, LY::Q_SOL, FAST ? q.br : q.il, rg);
+        stn(dst, LY::Q_SOL + 1, q.mu, rg);
+        if constexpr (!FAST) stn(dst, LY::Q_SOL + 2, q.is, rg);
+    };
+    auto sol_plane = [&](uint32_t dst, uint32_t p0, const S* co, const S* cr) {
+        sol_one(dst, p0, co, false);
+        if (ring_s) sol_one(dst, p0, cr, true);
     };
     // concentration of plane s at the own and ring points (a benign value
     // outside the domain, so that no logarithm there leaves the normal range)
-    auto load_c = [&](int s, S* co, S* cr) {
-        const bool zin = s >= 0 && s < nz;
-        const long long zo = (long long)s * pl;
+    auto load_c = [&](int s, const S* cz, S* co, S* cr, bool zin) {
 #pragma unroll
         for (int l = 0; l < L; ++l) {
-            co[l] = (zin && own[l]) ? c_in[col[l] + zo] : (S)0.02;
-            if (SOL) cr[l] = (zin && rin[l]) ? c_in[rcol[l] + zo] : (S)0.02;
+            co[l] = (zin && own[l]) ? cz[col[l]] : (S)0.02;
+            if (SOL) cr[l] = (zin && rin[l]) ? cz[rcol[l]] : (S)0.02;
         }
     };
-
-    // ---- the cell's flags (x / y parts; z parts are per plane) ----
-    const bool xin = x >= 1 && x <= nx - 2;    // T interior, phase source, solute interior
-    const bool xph = x >= 2 && x <= nx - 3;    // phase interior
-    const bool xone = x >= 3 && x <= nx - 4;   // sole preimage of itself
-    bool yin[L], yph[L], yone[L];
-    int xl = 0, xh = -1, yl[L], yh[L];
-    if (xin) fpre_range(x, nx, &xl, &xh);
-#pragma unroll
-    for (int l = 0; l < L; ++l) {
-        yin[l] = yv[l] >= 1 && yv[l] <= ny - 2;
-        yph[l] = yv[l] >= 2 && yv[l] <= ny - 3;
-        yone[l] = yv[l] >= 3 && yv[l] <= ny - 4;
-        yl[l] = 0;
-        yh[l] = -1;
-        if (yin[l]) fpre_range(yv[l], ny, &yl[l], &yh[l]);
-    }
-    // CTA-uniform: every column and row of the tile lies in [3, N-4]
-    const bool tile_int = x0 >= 3 && x0 + TX + 3 <= nx && y0 >= 3 && y0 + TY + 3 <= ny;
 
     // ---- prologue: planes zb-2 .. zb+3 in flight, nodes zb-1, zb ----
     if (lead) {
-        fence_proxy_async_smem();   // the slots may hold a previous tile's planes
         for (int p = zb - 2; p <= zb + 3; ++p)
             if (p >= 0 && p <= zlast) issue(p, (p + 6) % 6);
     }
-    S co[3][L], cr[2][L];   // concentration: own points of planes z, z+1, z+2; ring points of z+1, z+2
-    S nd[L], nt[L];         // centre values of the next plane: DPP (or the noise), TOLD
+    S co[L], c1[L], c2[L];      // concentration at the own points of planes z, z+1, z+2
+    S cr1[L], cr2[L];           // ... at the ring points of planes z+1, z+2
+    S nd[L], nt[L];             // centre values of the next plane: DPP (or the noise), TOLD
 #pragma unroll
-    for (int l = 0; l < L; ++l) { nd[l] = 0; nt[l] = 0; cr[0][l] = cr[1][l] = 0; }
+    for (int l = 0; l < L; ++l) nd[l] = nt[l] = c1[l] = c2[l] = cr1[l] = cr2[l] = 0;
     // DPP / noise and TOLD of the own cells of plane z.  TOLD is read only
     // where the heat equation keeps it (outside 2..N-1): inside, TNEW is TP
     // plus the latent term (and the Laplacian reads its own neighbours)
-    auto load_centre = [&](int z) {
-        if (!(HEAT || ran_mode == 2) || z >= ze) return;
-        const long long zo = (long long)z * pl;
-        const bool zi = z >= 1 && z <= nz - 2;
+    auto load_centre = [&](int z, long long zo, bool zi) {
+        if (!(HEAT || ran_mode == 2)) return;
+        const S* const dz = dpp + zo;
 #pragma unroll
         for (int l = 0; l < L; ++l) {
             if (!own[l]) continue;
-            nd[l] = dpp[col[l] + zo];
-            if (HEAT && !(zi && x >= 1 && x <= nx - 2 && yv[l] >= 1 && yv[l] <= ny - 2)) nt[l] = T_old[col[l] + zo];
+            nd[l] = dz[col[l]];
+            if (HEAT && !(zi && xyin[l])) nt[l] = (T_old + zo)[col[l]];
         }
     };
-    // rolled own-column state (window mode 5): phase values of planes z-1,
-    // z, z+1 at the cell and its N, S, E, W neighbours; the cell's node
-    // (eps^2, eyz, ezx) and solute-point (bracket, mu) quantities of the same
-    // planes.  Index of the five phase values: cell, N, S, E, W.  Unused, and
-    // so not allocated, in the other modes.
-    S rpm[L][5], rp0[L][5], rpp[L][5];
-    S rnB[L][3], rnC[L][3], rnT[L][3];
-    S rsB[L][2], rsP[L][2], rsT[L][2];
-    auto load5 = [&](S (*dst)[5], const S* pl_) {
-        if constexpr (ROLL) {
-#pragma unroll
-            for (int l = 0; l < L; ++l) {
-                const S* q = pl_ + phi_off[l];
-                dst[l][0] = q[0]; dst[l][1] = q[TW]; dst[l][2] = q[-TW]; dst[l][3] = q[1]; dst[l][4] = q[-1];
-            }
-        }
-    };
+    auto zin = [&](int z) { return z >= 1 && z <= nz - 2; };
+    auto zdom = [&](int z) { return z >= 0 && z < nz; };
     bool bad = false;
+    const long long zo0 = (long long)zb * pl;
+    auto wait_first = [&]() {
+        for (int p = zb - 2; p <= zb + 1; ++p)
+            if (p >= 0 && p <= zlast) bad |= !wait_plane((p + 6) % 6);
+    };
+    uint32_t n0 = node_at(0), np = node_at(1), nm = node_at(2);   // slots of planes z, z+1, z-1
     if (SOL) {
         S ca[L], cra[L];
-        load_c(zb - 1, ca, cra);
-        load_c(zb, co[0], cr[0]);
-        load_c(zb + 1, co[1], cr[1]);
-        for (int p = zb - 2; p <= zb + 1; ++p)
-            if (p >= 0 && p <= zlast) bad |= !wait_plane((p + 6) % 6);
-        if (zb - 1 >= 0)
-            sol_plane(wrap_add<NSLOT>(zb % NSLOT, NSLOT - 1), sphi + ((zb + 5) % 6) * LY::PHI_SLOT, ca, cra,
-                      ROLL ? rsB : nullptr, nullptr);
-        sol_plane(zb % NSLOT, sphi + (zb % 6) * LY::PHI_SLOT, co[0], cr[0], ROLL ? rsP : nullptr, nullptr);
-#pragma unroll
-        for (int l = 0; l < L; ++l) cr[0][l] = cr[1][l];
+        load_c(zb - 1, c_in + zo0 - pl, ca, cra, zdom(zb - 1));
+        load_c(zb, c_in + zo0, co, cr2, true);
+        load_c(zb + 1, c_in + zo0 + pl, c1, cr1, zdom(zb + 1));
+        wait_first();
+        if (zb - 1 >= 0) sol_plane(nm, phi_at((zb + 5) % 6), ca, cra);
+        sol_plane(n0, phi_at(zb % 6), co, cr2);
     } else {
-        load_c(zb, co[0], cr[0]);
-        for (int p = zb - 2; p <= zb + 1; ++p)
-            if (p >= 0 && p <= zlast) bad |= !wait_plane((p + 6) % 6);
+        load_c(zb, c_in + zo0, co, cr2, true);
+        wait_first();
     }
-    load_centre(zb);
-    if (PHASE && zb - 1 >= 1 && zb - 1 <= nz - 2)
-        node_plane(wrap_add<NSLOT>(zb % NSLOT, NSLOT - 1), sphi + ((zb + 4) % 6) * LY::PHI_SLOT,
-                   sphi + ((zb + 5) % 6) * LY::PHI_SLOT,
-                   sphi + (zb % 6) * LY::PHI_SLOT, ROLL ? rnB : nullptr);
-    if (PHASE && zb >= 1 && zb <= nz - 2)
-        node_plane(zb % NSLOT, sphi + ((zb + 5) % 6) * LY::PHI_SLOT, sphi + (zb % 6) * LY::PHI_SLOT,
-                   sphi + ((zb + 1) % 6) * LY::PHI_SLOT, ROLL ? rnC : nullptr);
-    load5(rpm, sphi + ((zb + 5) % 6) * LY::PHI_SLOT);
-    load5(rp0, sphi + (zb % 6) * LY::PHI_SLOT);
+    load_centre(zb, zo0, zin(zb));
+    if (PHASE && zin(zb - 1)) node_plane(nm, phi_at((zb + 4) % 6), phi_at((zb + 5) % 6), phi_at(zb % 6));
+    if (PHASE && zin(zb)) node_plane(n0, phi_at((zb + 5) % 6), phi_at(zb % 6), phi_at((zb + 1) % 6));
 
-    long long zoff = (long long)zb * pl;
     uint64_t hin[L];   // noise hash input of the own cells, carried along z (k = z + 1)
 #pragma unroll
-    for (int l = 0; l < L; ++l) hin[l] = hash_base(x + 1, yv[l] + 1, c.it, 1) + (uint64_t)(zb + 1) * kHashK;
-    int s6 = zb % 6;       // phase slot of plane z
-    int sn = zb % NSLOT;   // node / point slot of plane z
+    for (int l = 0; l < L; ++l)
+        hin[l] = hash_base(x0 + tx + 1, y0 + ty + l * TR + 1, c.it, 1) + (uint64_t)(zb + 1) * kHashK;
+    uint32_t am = phi_at((zb + 5) % 6), a0 = phi_at(zb % 6), ap = phi_at((zb + 1) % 6);   // planes z-1, z, z+1
+    int sq = (zb + 2) % 6;       // phase slot of plane z+2
+    long long zoff = zo0;
 
     // One plane of the march.  IN: every z-dependent condition of the plane
     // is known true (z in [3, N-4], the planes it reads and the load it
@@ -441,96 +380,47 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
     // stack (measured: 5x slower).
     auto plane = [&](int z, auto in_tag) __attribute__((always_inline)) -> bool {
         constexpr bool IN = decltype(in_tag)::value;
-        const int s6p1 = wrap_add<6>(s6, 1), s6p2 = wrap_add<6>(s6, 2);
-        const int snm1 = wrap_add<NSLOT>(sn, NSLOT - 1), snp1 = wrap_add<NSLOT>(sn, 1);
-        const S* const pm = sphi + wrap_add<6>(s6, 5) * LY::PHI_SLOT;
-        const S* const p0 = sphi + s6 * LY::PHI_SLOT;
-        const S* const pp = sphi + s6p1 * LY::PHI_SLOT;
-        const S* const pq = sphi + s6p2 * LY::PHI_SLOT;
+        const uint32_t aq = phi_at(sq);
         S dcur[L], tcur[L];
 #pragma unroll
         for (int l = 0; l < L; ++l) { dcur[l] = nd[l]; tcur[l] = nt[l]; }
-        load_centre(z + 1);
-        if (SOL) load_c(z + 2, co[2], cr[1]);
-        else load_c(z + 1, co[1], cr[1]);
+        if (IN || z + 1 < ze) load_centre(z + 1, zoff + pl, IN || zin(z + 1));
+        if (SOL) load_c(z + 2, c_in + zoff + 2 * pl, c2, cr2, IN || zdom(z + 2));
+        else load_c(z + 1, c_in + zoff + pl, c1, cr1, IN || zdom(z + 1));
 
         // A: plane z+2 has landed
-        if (IN || z + 2 <= zlast) bad |= !wait_plane(s6p2);
+        if (IN || z + 2 <= zlast) bad |= !wait_plane(sq);
         // B, C: nodes and solute points of plane z+1
-        if constexpr (ROLL) {
-            load5(rpp, pp);   // plane z+1 at the own column: the stencil's T values and the node's x/y gradient
-            if (IN || (z + 1 >= 1 && z + 1 <= nz - 2)) {
-                S a[L], b[L];
-#pragma unroll
-                for (int l = 0; l < L; ++l) { a[l] = rpp[l][3]; b[l] = rpp[l][4]; }
-                const V gx = grad<V, FAST>(LN::make(a), LN::make(b), cv.dx, cv.hx);
-#pragma unroll
-                for (int l = 0; l < L; ++l) { a[l] = rpp[l][1]; b[l] = rpp[l][2]; }
-                const V gy = grad<V, FAST>(LN::make(a), LN::make(b), cv.dy, cv.hy);
-#pragma unroll
-                for (int l = 0; l < L; ++l) { a[l] = pq[phi_off[l]]; b[l] = rp0[l][0]; }
-                const V gz = grad<V, FAST>(LN::make(a), LN::make(b), cv.dz, cv.hz);
-                S* const dst = snode + snp1 * LY::NODE_SLOT;
-                node_store(dst, node_off, gx, gy, gz, rnT);
-                if (ring) {
-#pragma unroll
-                    for (int l = 0; l < L; ++l) { a[l] = pp[rphi_off[l] + 1]; b[l] = pp[rphi_off[l] - 1]; }
-                    const V rx = grad<V, FAST>(LN::make(a), LN::make(b), cv.dx, cv.hx);
-#pragma unroll
-                    for (int l = 0; l < L; ++l) { a[l] = pp[rphi_off[l] + TW]; b[l] = pp[rphi_off[l] - TW]; }
-                    const V ry = grad<V, FAST>(LN::make(a), LN::make(b), cv.dy, cv.hy);
-#pragma unroll
-                    for (int l = 0; l < L; ++l) { a[l] = pq[rphi_off[l]]; b[l] = p0[rphi_off[l]]; }
-                    const V rz = grad<V, FAST>(LN::make(a), LN::make(b), cv.dz, cv.hz);
-                    node_store(dst, rnode_off, rx, ry, rz, nullptr);
-                }
-            }
-            if (SOL && (IN || z + 1 <= nz - 1)) {
-                S op[L];
-#pragma unroll
-                for (int l = 0; l < L; ++l) op[l] = rpp[l][0];
-                sol_plane(snp1, pp, co[1], cr[0], rsT, op);
-            }
-        } else {
-            if (PHASE && (IN || (z + 1 >= 1 && z + 1 <= nz - 2))) node_plane(snp1, p0, pp, pq, nullptr);
-            if (SOL && (IN || z + 1 <= nz - 1)) sol_plane(snp1, pp, co[1], cr[0], nullptr, nullptr);
-        }
+        if (PHASE && (IN || zin(z + 1))) node_plane(np, a0, ap, aq);
+        if (SOL && (IN || z + 1 <= nz - 1)) sol_plane(np, ap, c1, cr1);
         // D: one barrier orders the plane; everyone learns of a failed load
         if (__syncthreads_or(bad)) {
             drain();
             return false;
         }
-        // E: the load of plane z+4 into the slot plane z-2 has left
-        if (lead && (IN || z + 4 <= zlast)) {
-            fence_proxy_async_smem();
-            issue(z + 4, wrap_add<6>(s6, 4));
-        }
+        // E: the load of plane z+4 into the slot plane z-2 has left (read
+        // only, by threads that are behind the barrier)
+        if (lead && (IN || z + 4 <= zlast)) issue(z + 4, sq + 2 >= 6 ? sq - 4 : sq + 2);
 
         // F: the cells of plane z
-        const bool zin = IN || (z >= 1 && z <= nz - 2);   // T interior / phase source / solute interior
+        const bool zi = IN || zin(z);                     // T interior / phase source / solute interior
         const bool zph = IN || (z >= 2 && z <= nz - 3);   // phase interior
-        const S* const nm1 = snode + snm1 * LY::NODE_SLOT;
-        const S* const n0 = snode + sn * LY::NODE_SLOT;
-        const S* const np1 = snode + snp1 * LY::NODE_SLOT;
-        S PPs[L];
-#pragma unroll
-        for (int l = 0; l < L; ++l) PPs[l] = ROLL ? rp0[l][0] : p0[phi_off[l]];
-        const V PP = LN::make(PPs);
-        const V CPP = LN::make(co[0]);
+        const V PP = ldv(a0, 0, false);
+        const V CPP = LN::make(co);
 
-        // the REAL(4) noise of the own cells
-        float ran[L];
+        // the REAL(4) noise of the own cells, exact in S
+        S ran[L];
 #pragma unroll
         for (int l = 0; l < L; ++l) {
             if constexpr (!PHASE) {
-                ran[l] = 0.f;
+                ran[l] = (S)0;
             } else if constexpr (ran_mode == 2) {
-                ran[l] = (float)dcur[l];
+                ran[l] = dcur[l];
             } else if constexpr (SMOOTH) {
-                ran[l] = (c.rt == 2) ? phase_ran(2, x + 1, yv[l] + 1, z + 1, c.it)
-                                     : __double2float_rn(ran64(hash63_mix(hin[l])));
+                ran[l] = (S)((c.rt == 2) ? phase_ran(2, x0 + tx + 1, y0 + ty + l * TR + 1, z + 1, c.it)
+                                         : __double2float_rn(ran64(hash63_mix(hin[l]))));
             } else {
-                ran[l] = __double2float_rn(ran64(hash63_mix(hin[l])));
+                ran[l] = (S)__double2float_rn(ran64(hash63_mix(hin[l])));
             }
             hin[l] += kHashK;
         }
@@ -538,83 +428,38 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
         V ppn = PP;
         if (PHASE && zph) {
             Nbr<V> nb;
-            S t[L];
-#define PF3D_NB(FIELD, PLANE, DELTA)                                         \
-    _Pragma("unroll") for (int l = 0; l < L; ++l) t[l] = PLANE[phi_off[l] + (DELTA)]; \
-    nb.FIELD = LN::make(t);
-#define PF3D_NR(FIELD, ARR, I)                                               \
-    _Pragma("unroll") for (int l = 0; l < L; ++l) t[l] = ARR[l][I];          \
-    nb.FIELD = LN::make(t);
             nb.PP = PP;
-            if constexpr (ROLL) {
-                PF3D_NR(PN, rp0, 1) PF3D_NR(PS, rp0, 2) PF3D_NR(PE, rp0, 3) PF3D_NR(PW, rp0, 4)
-                PF3D_NR(PT, rpp, 0) PF3D_NR(PB, rpm, 0)
-                PF3D_NR(PNT, rpp, 1) PF3D_NR(PNB, rpm, 1) PF3D_NR(PST, rpp, 2) PF3D_NR(PSB, rpm, 2)
-                PF3D_NR(PET, rpp, 3) PF3D_NR(PEB, rpm, 3) PF3D_NR(PWT, rpp, 4) PF3D_NR(PWB, rpm, 4)
-            } else {
-                PF3D_NB(PN, p0, TW) PF3D_NB(PS, p0, -TW) PF3D_NB(PE, p0, 1) PF3D_NB(PW, p0, -1)
-                PF3D_NB(PT, pp, 0) PF3D_NB(PB, pm, 0)
-                PF3D_NB(PNT, pp, TW) PF3D_NB(PNB, pm, TW) PF3D_NB(PST, pp, -TW) PF3D_NB(PSB, pm, -TW)
-                PF3D_NB(PET, pp, 1) PF3D_NB(PEB, pm, 1) PF3D_NB(PWT, pp, -1) PF3D_NB(PWB, pm, -1)
-            }
-            PF3D_NB(PNE, p0, TW + 1) PF3D_NB(PSE, p0, -TW + 1) PF3D_NB(PNW, p0, TW - 1) PF3D_NB(PSW, p0, -TW - 1)
-#undef PF3D_NB
+            nb.PN = ldv(a0, PR, false); nb.PS = ldv(a0, -PR, false);
+            nb.PE = ldv(a0, ES, false); nb.PW = ldv(a0, -ES, false);
+            nb.PT = ldv(ap, 0, false); nb.PB = ldv(am, 0, false);
+            nb.PNT = ldv(ap, PR, false); nb.PNB = ldv(am, PR, false);
+            nb.PST = ldv(ap, -PR, false); nb.PSB = ldv(am, -PR, false);
+            nb.PET = ldv(ap, ES, false); nb.PEB = ldv(am, ES, false);
+            nb.PWT = ldv(ap, -ES, false); nb.PWB = ldv(am, -ES, false);
+            nb.PNE = ldv(a0, PR + ES, false); nb.PSE = ldv(a0, -PR + ES, false);
+            nb.PNW = ldv(a0, PR - ES, false); nb.PSW = ldv(a0, -PR - ES, false);
             Node<V> E, W, N, So, Tt, B;
-#define PF3D_ND(NODE, Q, PLANE, DELTA, QI)                                   \
-    _Pragma("unroll") for (int l = 0; l < L; ++l) t[l] = PLANE[node_off[l] + (DELTA) + (QI) * NQ]; \
-    NODE.Q = LN::make(t);
-            PF3D_ND(E, eps, n0, 1, 0) PF3D_ND(E, exy, n0, 1, 1) PF3D_ND(E, ezx, n0, 1, 3)
-            PF3D_ND(W, eps, n0, -1, 0) PF3D_ND(W, exy, n0, -1, 1) PF3D_ND(W, ezx, n0, -1, 3)
-            PF3D_ND(N, eps, n0, NW, 0) PF3D_ND(N, exy, n0, NW, 1) PF3D_ND(N, eyz, n0, NW, 2)
-            PF3D_ND(So, eps, n0, -NW, 0) PF3D_ND(So, exy, n0, -NW, 1) PF3D_ND(So, eyz, n0, -NW, 2)
-            if constexpr (ROLL) {
-#define PF3D_NN(NODE, Q, ARR, I)                                             \
-    _Pragma("unroll") for (int l = 0; l < L; ++l) t[l] = ARR[l][I];          \
-    NODE.Q = LN::make(t);
-                PF3D_NN(Tt, eps, rnT, 0) PF3D_NN(Tt, eyz, rnT, 1) PF3D_NN(Tt, ezx, rnT, 2)
-                PF3D_NN(B, eps, rnB, 0) PF3D_NN(B, eyz, rnB, 1) PF3D_NN(B, ezx, rnB, 2)
-#undef PF3D_NN
-            } else {
-                PF3D_ND(Tt, eps, np1, 0, 0) PF3D_ND(Tt, eyz, np1, 0, 2) PF3D_ND(Tt, ezx, np1, 0, 3)
-                PF3D_ND(B, eps, nm1, 0, 0) PF3D_ND(B, eyz, nm1, 0, 2) PF3D_ND(B, ezx, nm1, 0, 3)
-            }
-#undef PF3D_ND
-#undef PF3D_NR
+            E.eps = ldn(n0, ES); E.exy = ldn(n0, ES + NB); E.ezx = ldn(n0, ES + 3 * NB);
+            W.eps = ldn(n0, -ES); W.exy = ldn(n0, -ES + NB); W.ezx = ldn(n0, -ES + 3 * NB);
+            N.eps = ldn(n0, NR); N.exy = ldn(n0, NR + NB); N.eyz = ldn(n0, NR + 2 * NB);
+            So.eps = ldn(n0, -NR); So.exy = ldn(n0, -NR + NB); So.eyz = ldn(n0, -NR + 2 * NB);
+            Tt.eps = ldn(np, 0); Tt.eyz = ldn(np, 2 * NB); Tt.ezx = ldn(np, 3 * NB);
+            B.eps = ldn(nm, 0); B.eyz = ldn(nm, 2 * NB); B.ezx = ldn(nm, 3 * NB);
             E.eyz = W.eyz = N.ezx = So.ezx = Tt.exy = B.exy = V((S)0);   // unused by the body
-            S rs[L];
-#pragma unroll
-            for (int l = 0; l < L; ++l) rs[l] = (S)ran[l];
-            ppn = phase_ppnew<V, FAST, true>(nb, E, W, N, So, Tt, B, CPP, LN::make(rs), cv);
+            ppn = phase_ppnew<V, FAST, true, HQ>(nb, E, W, N, So, Tt, B, CPP, LN::make(ran), cv);
         }
         V cn = CPP;
-        if (SOL && zin) {
-            const S* const sm1 = ssol + snm1 * LY::SOL_SLOT;
-            const S* const s0 = ssol + sn * LY::SOL_SLOT;
-            const S* const sp1 = ssol + snp1 * LY::SOL_SLOT;
-            SolNode<V> q[7];   // P, E, W, N, S, T, B
-            S a[L], b[L];
-#define PF3D_SN(I, PLANE, DELTA)                                                                   \
-    _Pragma("unroll") for (int l = 0; l < L; ++l) { a[l] = PLANE[node_off[l] + (DELTA)];          \
-                                                     b[l] = PLANE[node_off[l] + (DELTA) + NQ]; }  \
-    q[I].br = q[I].il = LN::make(a);                                                               \
-    q[I].mu = LN::make(b);                                                                         \
-    if constexpr (!FAST) {                                                                         \
-        _Pragma("unroll") for (int l = 0; l < L; ++l) a[l] = PLANE[node_off[l] + (DELTA) + 2 * NQ]; \
-        q[I].is = LN::make(a);                                                                     \
-    }
-            PF3D_SN(1, s0, 1) PF3D_SN(2, s0, -1) PF3D_SN(3, s0, NW) PF3D_SN(4, s0, -NW)
-            if constexpr (ROLL) {
-#define PF3D_SR(I, ARR)                                                                              \
-    _Pragma("unroll") for (int l = 0; l < L; ++l) { a[l] = ARR[l][0]; b[l] = ARR[l][1]; }           \
-    q[I].br = LN::make(a);                                                                           \
-    q[I].mu = LN::make(b);
-                PF3D_SR(0, rsP) PF3D_SR(5, rsT) PF3D_SR(6, rsB)
-#undef PF3D_SR
-            } else {
-                PF3D_SN(0, s0, 0) PF3D_SN(5, sp1, 0) PF3D_SN(6, sm1, 0)
-            }
-#undef PF3D_SN
-            cn = conc_new<V, FAST>(PP, CPP, q[0], q[1], q[2], q[3], q[4], q[5], q[6], cv);
+        if (SOL && zi) {
+            constexpr int Q = LY::Q_SOL * NB;
+            auto sol_at = [&](uint32_t a, int off) {
+                SolNode<V> q;
+                q.br = q.il = ldn(a, off + Q);
+                q.mu = ldn(a, off + Q + NB);
+                if constexpr (!FAST) q.is = ldn(a, off + Q + 2 * NB);
+                return q;
+            };
+            cn = conc_new<V, FAST>(PP, CPP, sol_at(n0, 0), sol_at(n0, ES), sol_at(n0, -ES), sol_at(n0, NR),
+                                   sol_at(n0, -NR), sol_at(np, 0), sol_at(nm, 0), cv);
         }
         const V U = clamp01(ppn);
         const V DP = ppn - PP;
@@ -624,40 +469,43 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
             // preimage (CTA-uniform branch)
 #pragma unroll
             for (int l = 0; l < L; ++l) {
-                const long long id = col[l] + zoff;
-                if (HEAT) T_new[id] = heat_at<S>(T_old, id, px, pl, PPs[l], dcur[l], c);
-                if (ran_mode == 1) dpp[id] = (S)ran[l];
-                if (DPPW) dpp[id] = LN::get(DP, l);
-                if (PHASE) phi_out[id] = LN::get(U, l);
-                if (SOL) c_out[id] = LN::get(cn, l);
+                const uint32_t id = col[l];
+                if (HEAT) (T_new + zoff)[id] = heat_at<S, HQ>(T_old, zoff + id, px, pl, LN::get(PP, l), dcur[l], c);
+                if (ran_mode == 1) (dpp + zoff)[id] = ran[l];
+                if (DPPW) (dpp + zoff)[id] = LN::get(DP, l);
+                if (PHASE) (phi_out + zoff)[id] = LN::get(U, l);
+                if (SOL) (c_out + zoff)[id] = LN::get(cn, l);
             }
         } else {
 #pragma unroll
             for (int l = 0; l < L; ++l) {
                 if (!own[l]) continue;
-                const int y = yv[l];
-                const long long id = col[l] + zoff;
-                const bool src = xin && yin[l] && zin;   // T interior; phase copy source
+                const int x = x0 + tx, y = y0 + ty + l * TR;
+                const long long id = zoff + col[l];
+                const bool xin = x >= 1 && x <= nx - 2;          // T interior, phase source, solute interior
+                const bool src = xyin[l] && zi;                  // T interior; phase copy source
                 if (HEAT) {
                     S tn = tcur[l];
-                    if (src) tn = heat_at<S>(T_old, id, px, pl, PPs[l], dcur[l], c);
+                    if (src) tn = heat_at<S, HQ>(T_old, id, px, pl, LN::get(PP, l), dcur[l], c);
                     T_new[id] = tn;
                 }
                 if (PHASE && src) {
-                    const bool inner = xph && yph[l] && zph;
-                    S u = PPs[l];
+                    const bool inner = x >= 2 && x <= nx - 3 && y >= 2 && y <= ny - 3 && zph;
+                    S u = LN::get(PP, l);
                     if (inner) {
-                        if (ran_mode == 1) dpp[id] = (S)ran[l];
+                        if (ran_mode == 1) dpp[id] = ran[l];
                         if (DPPW) dpp[id] = LN::get(DP, l);
                         u = LN::get(U, l);
                     }
-                    if (xone && yone[l] && z >= 3 && z <= nz - 4) {
-                        phi_out[id] = u;
+                    if (x >= 3 && x <= nx - 4 && y >= 3 && y <= ny - 4 && z >= 3 && z <= nz - 4) {
+                        phi_out[id] = u;   // its own only preimage
                     } else {
-                        int zl, zh;
+                        int xl, xh, yl, yh, zl, zh;
+                        fpre_range(x, nx, &xl, &xh);
+                        fpre_range(y, ny, &yl, &yh);
                         fpre_range(z, nz, &zl, &zh);
                         for (int zz = zl; zz <= zh; ++zz)
-                            for (int yy = yl[l]; yy <= yh[l]; ++yy)
+                            for (int yy = yl; yy <= yh; ++yy)
                                 for (int xx = xl; xx <= xh; ++xx)
                                     phi_out[(long long)xx + (long long)yy * px + (long long)zz * pl] = u;
                     }
@@ -665,49 +513,35 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
                 if (SOL) {
                     // concentracao_soluto.f90:116-124 as a fan-out: the point
                     // writes its value to the face cells copied from it
-                    const S uc = src ? LN::get(cn, l) : co[0][l];
+                    const S uc = src ? LN::get(cn, l) : co[l];
                     if (src) c_out[id] = uc;
                     if (z == 1) c_out[id - pl] = uc;
                     if (z == nz - 2) c_out[id + pl] = uc;
-                    if (zin && x == 1) c_out[id - 1] = uc;
-                    if (zin && x == nx - 2) c_out[id + 1] = uc;
-                    if (zin && xin && y == 1) c_out[id - px] = uc;
-                    if (zin && xin && y == ny - 2) c_out[id + px] = uc;
+                    if (zi && x == 1) c_out[id - 1] = uc;
+                    if (zi && x == nx - 2) c_out[id + 1] = uc;
+                    if (zi && xin && y == 1) c_out[id - px] = uc;
+                    if (zi && xin && y == ny - 2) c_out[id + px] = uc;
                 }
             }
         }
 
-        // rotate the concentration registers and the phase slot
+        // the next plane's view of the windows and the carried concentrations
 #pragma unroll
         for (int l = 0; l < L; ++l) {
-            co[0][l] = co[1][l];
+            co[l] = c1[l];
             if (SOL) {
-                co[1][l] = co[2][l];
-                cr[0][l] = cr[1][l];
+                c1[l] = c2[l];
+                cr1[l] = cr2[l];
             }
         }
-        if constexpr (ROLL) {
-#pragma unroll
-            for (int l = 0; l < L; ++l) {
-#pragma unroll
-                for (int i = 0; i < 5; ++i) {
-                    rpm[l][i] = rp0[l][i];
-                    rp0[l][i] = rpp[l][i];
-                }
-#pragma unroll
-                for (int i = 0; i < 3; ++i) {
-                    rnB[l][i] = rnC[l][i];
-                    rnC[l][i] = rnT[l][i];
-                }
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {
-                    rsB[l][i] = rsP[l][i];
-                    rsP[l][i] = rsT[l][i];
-                }
-            }
-        }
-        s6 = s6p1;
-        sn = snp1;
+        am = a0;
+        a0 = ap;
+        ap = aq;
+        sq = sq == 5 ? 0 : sq + 1;
+        const uint32_t t = nm;
+        nm = n0;
+        n0 = np;
+        np = t;
         zoff += pl;
         return true;
     };
@@ -728,22 +562,39 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
     return true;
 }
 
+// The tile in the copy of the body that its position in the domain needs.  The
+// FP32 passes, with twice the CTAs in flight and half the instructions a cell,
+// are short of instruction cache and run the one copy with all its checks
+// (256^3: 668 us a step with interior copies of tiles and planes, 561 without;
+// FP64 340x340x200: 1290 us with, 1405 without).
+template <typename S, int L, int TY, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool SPLIT, bool PHASE, bool FAST,
+          int HQ>
+__device__ __forceinline__ bool march_any(const DomainDesc& d, const KC<S>& c, const KC<typename Lanes<S, L>::V>& cv,
+                                          const CUtensorMap* tm, const S* c_in, S* phi_out, S* dpp, S* c_out,
+                                          const S* T_old, S* T_new, int zchunk, int bx, int by, int bz,
+                                          unsigned char* smem, uint32_t& par)
+{
+    const int x0 = bx * 32, y0 = by * TY;
+    constexpr bool copies = sizeof(S) == 8;
+    if (copies && x0 >= 3 && x0 + 32 + 3 <= d.nx && y0 >= 3 && y0 + TY + 3 <= d.ny)
+        return march_tile<S, L, TY, HEAT, DPPW, SOL, SMOOTH, SPLIT, PHASE, FAST, HQ, true>(
+            d, c, cv, tm, c_in, phi_out, dpp, c_out, T_old, T_new, zchunk, bx, by, bz, smem, par);
+    return march_tile<S, L, TY, HEAT, DPPW, SOL, SMOOTH, SPLIT, PHASE, FAST, HQ, false>(
+        d, c, cv, tm, c_in, phi_out, dpp, c_out, T_old, T_new, zchunk, bx, by, bz, smem, par);
+}
+
 // resident CTAs per SM the register budget is sized for (shared memory
-// allows no more): FP64 3, or 2 -- 128 registers a thread -- for the rolled
-// window mode (its carried column values), a solute pass with 4-plane
-// windows and a pass that may draw the smooth noise (its trilinear blend of
-// eight hashes); FP32 pairs 6 (80 registers, no spills), 5 in the rolled
-// mode; FP32 single cells 3
-template <typename S, int L, int WIN, bool SOL, bool HEAT, bool SMOOTH = false>
+// allows no more): FP64 3 (80 registers a thread), or 2 for a pass that may
+// draw the smooth noise (its trilinear blend of eight hashes) and for the
+// reference form of the sweep; FP32 pairs 6, FP32 single cells 3
+template <typename S, int L, bool SMOOTH, bool PHASE = true, bool FAST = true>
 struct MarchOcc {
-    static constexpr int v = (sizeof(S) == 8) ? ((WIN == 5 || (SOL && WIN == 4) || SMOOTH) ? 2 : 3)
-                                              : (L == 2 ? ((WIN != 5) ? 6 : 5) : 3);
+    static constexpr int v = (sizeof(S) == 8) ? ((SMOOTH || (PHASE && !FAST)) ? 2 : 3) : (L == 2 ? 6 : 3);
 };
 
 // single domain: one CTA per tile; the phase field comes through `tm`
-template <typename S, int L, int TY, int WIN, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool PHASE = true,
-          bool FAST = true>
-__global__ void __launch_bounds__(32 * TY / L, (FAST ? MarchOcc<S, L, WIN, SOL, HEAT, SMOOTH>::v : PHASE ? 2 : 3))
+template <typename S, int L, int TY, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool PHASE, bool FAST, int HQ>
+__global__ void __launch_bounds__(32 * TY / L, (MarchOcc<S, L, SMOOTH, PHASE, FAST>::v))
     k_march(const __grid_constant__ CUtensorMap tm, DomainDesc d, const KC<S> c,
             const KC<typename Lanes<S, L>::V> cv, const S* __restrict__ c_in, S* __restrict__ phi_out,
             S* __restrict__ dpp, S* __restrict__ c_out, const S* __restrict__ T_old, S* __restrict__ T_new,
@@ -751,11 +602,11 @@ __global__ void __launch_bounds__(32 * TY / L, (FAST ? MarchOcc<S, L, WIN, SOL, 
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* smem = align128(smem_raw);
-    march_init_barriers<MarchLayout<S, TY, SOL, MarchWin<WIN>::nslot, PHASE, FAST>>(smem);
+    march_init_barriers<MarchLayout<S, TY, SOL, PHASE, FAST>>(smem);
     uint32_t par = 0;
-    if (!march_tile<S, L, TY, WIN, HEAT, DPPW, SOL, SMOOTH, true, PHASE, FAST>(d, c, cv, &tm, c_in, phi_out, dpp, c_out, T_old,
-                                                                T_new, zchunk, blockIdx.x, blockIdx.y, blockIdx.z,
-                                                                smem, par)) {
+    if (!march_any<S, L, TY, HEAT, DPPW, SOL, SMOOTH, sizeof(S) == 8, PHASE, FAST, HQ>(
+            d, c, cv, &tm, c_in, phi_out, dpp, c_out, T_old, T_new, zchunk, blockIdx.x, blockIdx.y, blockIdx.z, smem,
+            par)) {
         if (threadIdx.x == 0 && threadIdx.y == 0) atomicExch(err, kErrTmaTimeout);
     }
 }
@@ -769,9 +620,8 @@ __global__ void __launch_bounds__(32 * TY / L, (FAST ? MarchOcc<S, L, WIN, SOL, 
 // counter *ctr (zero before the launch), so CTAs that drew short items (thin
 // z-chunks, small domains at the end of the largest-first list) keep
 // working while others finish long ones.
-template <typename S, int L, int TY, int WIN, int PASS, bool ONE_SWEEP, bool SMOOTH>
-__global__ void __launch_bounds__(32 * TY / L,
-                                  (MarchOcc<S, L, WIN, PASS == 1 || ONE_SWEEP, PASS == 0, SMOOTH>::v))
+template <typename S, int L, int TY, int PASS, bool ONE_SWEEP, bool SMOOTH>
+__global__ void __launch_bounds__(32 * TY / L, (MarchOcc<S, L, SMOOTH>::v))
     k_march_batch(const BatchDomain* __restrict__ doms, const CUtensorMap* __restrict__ tmaps,
                   const BatchStep* __restrict__ steps, const BatchItem* __restrict__ items,
                   const int* __restrict__ head, int* __restrict__ ctr, int* __restrict__ err)
@@ -785,7 +635,7 @@ __global__ void __launch_bounds__(32 * TY / L,
     constexpr int nf = (int)(offsetof(KC<S>, hq) / sizeof(S));
     constexpr int NT = 32 * TY / L;
     unsigned char* smem = align128(smem_raw);
-    march_init_barriers<MarchLayout<S, TY, SOL, MarchWin<WIN>::nslot>>(smem);
+    march_init_barriers<MarchLayout<S, TY, SOL>>(smem);
     uint32_t par = 0;
     const int n = head[0], zchunk = head[1];
     const int tid = threadIdx.x + 32 * threadIdx.y;
@@ -823,16 +673,16 @@ __global__ void __launch_bounds__(32 * TY / L,
         if (PASS == 0) {
             const CUtensorMap* tm = tmaps + 2 * it.dom + q;
             if (ONE_SWEEP)
-                ok = march_tile<S, L, TY, WIN, true, true, true, SMOOTH, false>(
+                ok = march_any<S, L, TY, true, true, true, SMOOTH, false, true, true, 2>(
                     D.d, skc, kv, tm, (const S*)D.c[qc], (S*)D.phi[1 - q], (S*)D.dpp, (S*)D.c[1 - qc],
                     (const S*)D.T[qt], (S*)D.T[1 - qt], zchunk, it.bx, it.by, it.bz, smem, par);
             else
-                ok = march_tile<S, L, TY, WIN, true, false, false, SMOOTH, false>(
+                ok = march_any<S, L, TY, true, false, false, SMOOTH, false, true, true, 2>(
                     D.d, skc, kv, tm, (const S*)D.c[qc], (S*)D.phi[1 - q], (S*)D.dpp, nullptr, (const S*)D.T[qt],
                     (S*)D.T[1 - qt], zchunk, it.bx, it.by, it.bz, smem, par);
         } else {
             const CUtensorMap* tm = tmaps + 2 * it.dom + (1 - q);
-            ok = march_tile<S, L, TY, WIN, false, true, true, false, false>(
+            ok = march_any<S, L, TY, false, true, true, false, false, true, true, 2>(
                 D.d, skc, kv, tm, (const S*)D.c[qc], (S*)D.phi[q], (S*)D.dpp, (S*)D.c[1 - qc], nullptr, nullptr,
                 zchunk, it.bx, it.by, it.bz, smem, par);
         }
@@ -871,14 +721,13 @@ KC<typename Lanes<S, L>::V> kc_lanes(const KC<S>& k)
     }
 }
 
-template <typename S, int L, int TY, int WIN, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool PHASE = true,
-          bool FAST = true>
+template <typename S, int L, int TY, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool PHASE, bool FAST, int HQ>
 cudaError_t launch_march_t(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s, const void* c_in,
                            void* phi_out, void* dpp, void* c_out, const void* T_old, void* T_new, int zchunk,
                            int* err, cudaStream_t st)
 {
-    using LY = MarchLayout<S, TY, SOL, MarchWin<WIN>::nslot, PHASE, FAST>;
-    auto kern = k_march<S, L, TY, WIN, HEAT, DPPW, SOL, SMOOTH, PHASE, FAST>;
+    using LY = MarchLayout<S, TY, SOL, PHASE, FAST>;
+    auto kern = k_march<S, L, TY, HEAT, DPPW, SOL, SMOOTH, PHASE, FAST, HQ>;
     static bool configured = false;   // one attribute call per instantiation
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::ALLOC);
@@ -895,36 +744,33 @@ cudaError_t launch_march_t(const CUtensorMap& tm, const DomainDesc& d, const Ste
     return cudaGetLastError();
 }
 
-// the passes of a step (32 x 8 tiles).  lanes: cells per thread (1 or 2);
-// win: window mode (3, 4 or 5, MarchWin).  The smooth noise runs one cell
-// per thread.
+// the passes of a step (32 x 8 tiles).  lanes: cells per thread (1 or 2); the
+// smooth noise runs one cell per thread.  h(phi) is known at compile time.
 template <typename S>
 cudaError_t launch_march_first(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s, const Fields& f,
-                               bool with_solute, int lanes, int win, int zchunk, int* err, cudaStream_t st)
+                               bool with_solute, int lanes, int zchunk, int* err, cudaStream_t st)
 {
-    const bool smooth = d.rt == 2;
-#define PF3D_MF(L, NS, DW, SO, SM)                                                                            \
-    launch_march_t<S, L, 8, NS, true, DW, SO, SM>(tm, d, s, f.c_old, f.phi_mid, f.dpp, SO ? f.c_new : nullptr, \
-                                                  f.T_old, f.T_new, zchunk, err, st)
-#define PF3D_MW(L, DW, SO, SM) \
-    (win == 3 ? PF3D_MF(L, 3, DW, SO, SM) : win == 4 ? PF3D_MF(L, 4, DW, SO, SM) : PF3D_MF(L, 5, DW, SO, SM))
-    if (smooth) return with_solute ? PF3D_MW(1, true, true, true) : PF3D_MW(1, false, false, true);
-    if (with_solute) return lanes == 2 ? PF3D_MW(2, true, true, false) : PF3D_MW(1, true, true, false);
-    return lanes == 2 ? PF3D_MW(2, false, false, false) : PF3D_MW(1, false, false, false);
-#undef PF3D_MW
+#define PF3D_MF(L, SO, SM, HQ)                                                                                  \
+    launch_march_t<S, L, 8, true, SO, SO, SM, true, true, HQ>(tm, d, s, f.c_old, f.phi_mid, f.dpp,              \
+                                                              SO ? f.c_new : nullptr, f.T_old, f.T_new, zchunk, \
+                                                              err, st)
+#define PF3D_MQ(L, SO) (d.hq ? PF3D_MF(L, SO, false, 1) : PF3D_MF(L, SO, false, 0))
+    if (d.rt == 2) return with_solute ? PF3D_MF(1, true, true, 2) : PF3D_MF(1, false, true, 2);
+    if (with_solute) return lanes == 2 ? PF3D_MQ(2, true) : PF3D_MQ(1, true);
+    return lanes == 2 ? PF3D_MQ(2, false) : PF3D_MQ(1, false);
+#undef PF3D_MQ
 #undef PF3D_MF
 }
 
 template <typename S>
 cudaError_t launch_march_last(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s, const Fields& f,
-                              int lanes, int win, int zchunk, int* err, cudaStream_t st)
+                              int lanes, int zchunk, int* err, cudaStream_t st)
 {
-#define PF3D_ML(L, NS)                                                                                     \
-    launch_march_t<S, L, 8, NS, false, true, true, false>(tm, d, s, f.c_old, f.phi_new, f.dpp, f.c_new, nullptr, \
-                                                          nullptr, zchunk, err, st)
-#define PF3D_MW(L) (win == 3 ? PF3D_ML(L, 3) : win == 4 ? PF3D_ML(L, 4) : PF3D_ML(L, 5))
-    return lanes == 2 ? PF3D_MW(2) : PF3D_MW(1);
-#undef PF3D_MW
+#define PF3D_ML(L, HQ)                                                                                          \
+    launch_march_t<S, L, 8, false, true, true, false, true, true, HQ>(tm, d, s, f.c_old, f.phi_new, f.dpp,     \
+                                                                      f.c_new, nullptr, nullptr, zchunk, err, st)
+    if (lanes == 2) return d.hq ? PF3D_ML(2, 1) : PF3D_ML(2, 0);
+    return d.hq ? PF3D_ML(1, 1) : PF3D_ML(1, 0);
 #undef PF3D_ML
 }
 
@@ -942,7 +788,9 @@ cudaError_t launch_march_sweep(const CUtensorMap& tm, const DomainDesc& d, const
 {
     constexpr bool FAST = sizeof(S) == 4;
     const bool smooth = d.rt == 2;
-#define PF3D_MS(DW, SM)                                                                                                 launch_march_t<S, 1, 8, 3, false, DW, false, SM, true, FAST>(tm, d, s, c_in, phi_out, dpp, nullptr, nullptr,                                                                     nullptr, zchunk, err, st)
+#define PF3D_MS(DW, SM)                                                                                          \
+    launch_march_t<S, 1, 8, false, DW, false, SM, true, FAST, 2>(tm, d, s, c_in, phi_out, dpp, nullptr, nullptr, \
+                                                                 nullptr, zchunk, err, st)
     if (dpp) return smooth ? PF3D_MS(true, true) : PF3D_MS(true, false);
     return smooth ? PF3D_MS(false, true) : PF3D_MS(false, false);
 #undef PF3D_MS
@@ -952,20 +800,20 @@ template <typename S>
 cudaError_t launch_march_solute(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s, const void* c_in,
                                 void* c_out, int zchunk, int* err, cudaStream_t st)
 {
-    return launch_march_t<S, 1, 8, 3, false, false, true, false, false, sizeof(S) == 4>(
+    return launch_march_t<S, 1, 8, false, false, true, false, false, sizeof(S) == 4, 2>(
         tm, d, s, c_in, nullptr, nullptr, c_out, nullptr, nullptr, zchunk, err, st);
 }
 
 // The persistent grid is the SM count times the CTAs of this kernel that are
 // resident on one SM.
-template <typename S, int L, int WIN, int PASS, bool ONE_SWEEP, bool SMOOTH>
+template <typename S, int L, int PASS, bool ONE_SWEEP, bool SMOOTH>
 cudaError_t launch_march_batch_t(const BatchDomain* doms, const CUtensorMap* tmaps, const BatchStep* steps,
                                  const BatchItem* items, const int* head, int n_sm, int* ctr, int* err,
                                  cudaStream_t st)
 {
     constexpr bool SOL = PASS == 1 || ONE_SWEEP;
-    using LY = MarchLayout<S, 8, SOL, MarchWin<WIN>::nslot>;
-    auto kern = k_march_batch<S, L, 8, WIN, PASS, ONE_SWEEP, SMOOTH>;
+    using LY = MarchLayout<S, 8, SOL>;
+    auto kern = k_march_batch<S, L, 8, PASS, ONE_SWEEP, SMOOTH>;
     static int per_sm = 0;   // one attribute and occupancy query per instantiation
     if (per_sm == 0) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::ALLOC);
@@ -982,19 +830,16 @@ cudaError_t launch_march_batch_t(const BatchDomain* doms, const CUtensorMap* tma
 template <typename S>
 cudaError_t launch_march_batch(const BatchDomain* doms, const CUtensorMap* tmaps, const BatchStep* steps,
                                const BatchItem* items, const int* head, int pass, bool one_sweep, bool smooth,
-                               int lanes, int win, int n_sm, int* ctr, int* err, cudaStream_t st)
+                               int lanes, int n_sm, int* ctr, int* err, cudaStream_t st)
 {
-#define PF3D_MB(L, NS, P, ONE, SM) \
-    launch_march_batch_t<S, L, NS, P, ONE, SM>(doms, tmaps, steps, items, head, n_sm, ctr, err, st)
-#define PF3D_MW(L, P, ONE, SM) \
-    (win == 3 ? PF3D_MB(L, 3, P, ONE, SM) : win == 4 ? PF3D_MB(L, 4, P, ONE, SM) : PF3D_MB(L, 5, P, ONE, SM))
+#define PF3D_MB(L, P, ONE, SM) \
+    launch_march_batch_t<S, L, P, ONE, SM>(doms, tmaps, steps, items, head, n_sm, ctr, err, st)
     if (pass == 0) {
-        if (smooth) return one_sweep ? PF3D_MW(1, 0, true, true) : PF3D_MW(1, 0, false, true);
-        if (lanes == 2) return one_sweep ? PF3D_MW(2, 0, true, false) : PF3D_MW(2, 0, false, false);
-        return one_sweep ? PF3D_MW(1, 0, true, false) : PF3D_MW(1, 0, false, false);
+        if (smooth) return one_sweep ? PF3D_MB(1, 0, true, true) : PF3D_MB(1, 0, false, true);
+        if (lanes == 2) return one_sweep ? PF3D_MB(2, 0, true, false) : PF3D_MB(2, 0, false, false);
+        return one_sweep ? PF3D_MB(1, 0, true, false) : PF3D_MB(1, 0, false, false);
     }
-    return lanes == 2 ? PF3D_MW(2, 1, false, false) : PF3D_MW(1, 1, false, false);
-#undef PF3D_MW
+    return lanes == 2 ? PF3D_MB(2, 1, false, false) : PF3D_MB(1, 1, false, false);
 #undef PF3D_MB
 }
 
