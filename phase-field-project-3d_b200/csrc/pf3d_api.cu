@@ -260,19 +260,18 @@ int pf_set_state(pf_ctx* ctx, const pf_state* st)
 // kernel reported a failure (the word is cleared after it is reported)
 static int kernel_status(pf_ctx* ctx)
 {
-    int code = 0;
-    CK(cudaMemcpyAsync(&code, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "status read");
+    int* const code = (int*)(ctx->h_out + 7);   // pinned: the copy rides on the one wait
+    CK(cudaMemcpyAsync(code, ctx->d_status, sizeof(int), cudaMemcpyDeviceToHost, ctx->stream), "status read");
     CK(cudaStreamSynchronize(ctx->stream), "status read");
-    if (code == 0) return PF_OK;
+    if (*code == 0) return PF_OK;
     CK(cudaMemsetAsync(ctx->d_status, 0, sizeof(int), ctx->stream), "status reset");
-    return ctx_err(ctx, PF_E_KERNEL, "a kernel reported failure code " + std::to_string(code) +
-                                         (code == kErrTmaTimeout ? " (a TMA plane load did not arrive in time)" : ""));
+    return ctx_err(ctx, PF_E_KERNEL, "a kernel reported failure code " + std::to_string(*code) +
+                                         (*code == kErrTmaTimeout ? " (a TMA plane load did not arrive in time)" : ""));
 }
 
 int pf_sync(pf_ctx* ctx)
 {
     if (!ctx) return PF_E_ARG;
-    CK(cudaStreamSynchronize(ctx->stream), "pf_sync");
     return kernel_status(ctx);
 }
 
@@ -399,7 +398,6 @@ int pf_download(pf_ctx* ctx, int field, double* host)
                "pf_download copy");
         }
     }
-    CK(cudaStreamSynchronize(ctx->stream), "pf_download sync");
     return kernel_status(ctx);
 }
 
@@ -514,13 +512,13 @@ int pf_auxiliar(const pf_ctx* ctx, double TP, double Cs_eq, double Cl_eq, double
 static int run_diag(pf_ctx* ctx, const void* phi, const void* c, const void* Tw, double out[5])
 {
     const void* dp = ctx->fld[PF_DPP];
-    CK(is64(ctx) ? launch_diag<double>(ctx->dd, phi, c, Tw, dp, ctx->d_part, ctx->nblk, ctx->d_out, ctx->stream)
-                 : launch_diag<float>(ctx->dd, phi, c, Tw, dp, ctx->d_part, ctx->nblk, ctx->d_out, ctx->stream),
+    CK(is64(ctx) ? launch_diag<double>(ctx->dd, phi, c, Tw, dp, ctx->d_part, ctx->d_out, ctx->stream)
+                 : launch_diag<float>(ctx->dd, phi, c, Tw, dp, ctx->d_part, ctx->d_out, ctx->stream),
        "diagnosticos");
     CK(cudaMemcpyAsync(ctx->h_out, ctx->d_out, 6 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream), "diag copy");
-    CK(cudaStreamSynchronize(ctx->stream), "diag sync");
+    const int rc = kernel_status(ctx);   // waits for the stream
+    if (rc == PF_E_CUDA) return rc;
     std::memcpy(out, ctx->h_out, 5 * sizeof(double));
-    const int rc = kernel_status(ctx);
     if (rc != PF_OK) return rc;
     if (ctx->h_out[5] != 0.0)
         return ctx_err(ctx, PF_E_NONFINITE, "diagnosticos: " + std::to_string((long long)ctx->h_out[5]) +

@@ -405,6 +405,7 @@ int pf_batch_create(int precision, long long budget_bytes, int max_domains, pf_b
     cudaMemset(b->d_steps, 0, step_bytes);
     cudaMemset(b->d_nitems, 0, 2 * sizeof(int));
     cudaMemset(b->d_status, 0, sizeof(int));
+    cudaMemset(b->d_part, 0, (592 * kDiagRow + 8) * sizeof(double));   // the diagnostics' block counter among it
     if (!tmap_encoder()) b->march = 0;   // no tensor-map encoder in this driver: the cp.async passes
     set_grid(b);
     *out = b;
@@ -739,13 +740,13 @@ int pf_batch_step_async(pf_batch* b, int n_steps)
 // kernel reported a failure (cleared once reported)
 static int batch_status(pf_batch* b)
 {
-    int code = 0;
-    BCK(cudaMemcpyAsync(&code, b->d_status, sizeof(int), cudaMemcpyDeviceToHost, b->stream), "status read");
+    int* const code = (int*)(b->h_out + 7);   // pinned: the copy rides on the one wait
+    BCK(cudaMemcpyAsync(code, b->d_status, sizeof(int), cudaMemcpyDeviceToHost, b->stream), "status read");
     BCK(cudaStreamSynchronize(b->stream), "status read");
-    if (code == 0) return PF_OK;
+    if (*code == 0) return PF_OK;
     BCK(cudaMemsetAsync(b->d_status, 0, sizeof(int), b->stream), "status reset");
-    return berr(b, PF_E_KERNEL, "a batch kernel reported failure code " + std::to_string(code) +
-                                    (code == kErrTmaTimeout ? " (a TMA plane load did not arrive in time)" : ""));
+    return berr(b, PF_E_KERNEL, "a batch kernel reported failure code " + std::to_string(*code) +
+                                    (*code == kErrTmaTimeout ? " (a TMA plane load did not arrive in time)" : ""));
 }
 
 // Waits for the steps of the last pf_batch_step_async; their device time is
@@ -912,14 +913,14 @@ int pf_batch_diagnosticos(pf_batch* b, int slot, double out[5])
     if (!sl || !out) return berr(b, PF_E_ARG, "pf_batch_diagnosticos: bad argument");
     double* res = b->d_part + 592 * kDiagRow;
     cudaError_t e = b64(b) ? launch_diag<double>(sl->bd.d, slot_field(*sl, PF_PHASE_OLD), slot_field(*sl, PF_CONC_OLD),
-                                                 slot_field(*sl, PF_TOLD), sl->bd.dpp, b->d_part, 592, res, b->stream)
+                                                 slot_field(*sl, PF_TOLD), sl->bd.dpp, b->d_part, res, b->stream)
                            : launch_diag<float>(sl->bd.d, slot_field(*sl, PF_PHASE_OLD), slot_field(*sl, PF_CONC_OLD),
-                                                slot_field(*sl, PF_TOLD), sl->bd.dpp, b->d_part, 592, res, b->stream);
+                                                slot_field(*sl, PF_TOLD), sl->bd.dpp, b->d_part, res, b->stream);
     BCK(e, "pf_batch_diagnosticos");
     BCK(cudaMemcpyAsync(b->h_out, res, 6 * sizeof(double), cudaMemcpyDeviceToHost, b->stream), "diag copy");
-    BCK(cudaStreamSynchronize(b->stream), "diag sync");
+    const int rc = batch_status(b);   // waits for the stream
+    if (rc == PF_E_CUDA) return rc;
     std::memcpy(out, b->h_out, 5 * sizeof(double));
-    const int rc = batch_status(b);
     if (rc != PF_OK) return rc;
     if (b->h_out[5] != 0.0)
         return berr(b, PF_E_NONFINITE, "pf_batch_diagnosticos: " + std::to_string((long long)b->h_out[5]) +

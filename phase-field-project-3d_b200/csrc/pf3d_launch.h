@@ -109,14 +109,14 @@ template <typename T> cudaError_t launch_shift_frame(const DomainDesc& d, int kd
                                                      void* phi_n, void* c_n, cudaStream_t st);
 template <typename T> cudaError_t launch_fill(void* a, long long n, double v, cudaStream_t st);
 
-// Diagnostics: block partials into part[nblk*kDiagRow], final into out[6]:
-// the five values of diagnosticos and the count of cells whose phi or c is
-// not finite (the watchdog).
+// Diagnostics: block partials into part[592*kDiagRow], result into out[8]: the
+// five values of diagnosticos, the count of cells whose phi, c, T or DPP is not
+// finite (the watchdog), and the kernel's own counter in the last double (zero
+// before the first call).  Tw and dpp (may be null): the temperature and DPP
+// fields the watchdog also checks.
 constexpr int kDiagRow = 10;   // l2, l2 comp, max, min, sol, sol comp, fe, fe comp, non-finite cells, pad
-// Tw and dpp (may be null): the temperature and DPP fields the watchdog
-// also checks for non-finite values.
 template <typename T> cudaError_t launch_diag(const DomainDesc& d, const void* phi, const void* c, const void* Tw,
-                                              const void* dppw, double* part, int nblk, double* out, cudaStream_t st);
+                                              const void* dppw, double* part, double* out, cudaStream_t st);
 
 // FP64 host array (Fortran order, nx*ny*nz) <-> pitched device field of T,
 // through a device staging buffer of doubles (FP32 contexts only).

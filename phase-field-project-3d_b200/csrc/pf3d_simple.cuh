@@ -103,43 +103,89 @@ struct KSum {
     }
 };
 
-// The grid walks 32 x 8-column tiles, each marched along z over a chunk of
-// kDiagZ planes (a persistent grid: block b takes tiles b, b + gridDim.x,
-// ...; the per-thread sums carry across its tiles, so the reduction order is
-// fixed by the launch shape).  The march goes in groups of kDiagG planes: a
-// thread first issues the reads of the whole group -- phi of the next
-// kDiagG planes and c, T, DPP of the group's planes, each cell read once from
-// HBM, all in flight together -- then shares the group's phase planes
-// through shared memory (one barrier a group) and evaluates its cells, with
-// the phase field of the planes above and below in registers (indexed at
-// compile time, so no register is moved before its load lands).  Only the
-// tile's edge cells read an in-plane neighbour from global memory (L2).  The
-// central gradient multiplies by the host-rounded 0.5/dx (within an ulp of
-// diag_body.inc's (a-b)*0.5d0/dx, far inside the sums' tolerance).  Within
-// a tile a thread sums its column's at most kDiagZ terms in plain FP64
-// (every term is nonnegative: phi^2, c and the energy density, so the
-// relative error stays below kDiagZ ulps) and adds the column sum to its
-// compensated (Neumaier) totals.
+// whether a value is NaN or infinite, from its bits
+__device__ __forceinline__ bool not_finite(double v) { return (__double2hiint(v) & 0x7ff00000) == 0x7ff00000; }
+__device__ __forceinline__ bool not_finite(float v) { return (__float_as_uint(v) & 0x7f800000u) == 0x7f800000u; }
+
+// The grid walks 32 x 8-column tiles, each marched along z over a chunk of zlen
+// planes (a persistent grid: block b takes tiles b, b + gridDim.x, ...; the
+// per-thread sums carry across its tiles, so the reduction order is fixed by
+// the launch shape).  The march goes in groups of kDiagG planes: a thread
+// first issues the reads of the whole group -- phi of the next kDiagG planes
+// and c, T, DPP of the group's planes, each cell read once from HBM, all in
+// flight together -- then shares the group's phase planes through shared
+// memory (one barrier a group) and evaluates its cells, with the phase field
+// of the planes above and below in registers (indexed at compile time, so no
+// register is moved before its load lands).
+//
+// FP64 arithmetic bounds the pass where memory does not (FP32 fields, small
+// domains), so a cell contributes bare squares -- phi^2, the three squared
+// central differences and (phi (1-phi))^2, eleven operations -- and the
+// factors of diag_body.inc (0.5 E0^2, (0.5/dx)^2, W0, dx dy dz) multiply the
+// column's sums once.  T and DPP, which only the watchdog reads, are tested
+// on their bits and never converted.  A column's at most kDiagZ terms are
+// summed in plain FP64 (every term is nonnegative: phi^2, c and the energy's
+// parts, so the relative error stays below kDiagZ ulps) and the column sums go
+// into compensated (Neumaier) totals.
+//
+// The last block to finish merges the blocks' partials (block order, fixed), so
+// the whole reduction is one launch.  pf_diagnosticos, call to answer, before and
+// after: 340x340x700 FP64 768 -> 488 us (5.3 TB/s, 0.81 of the measured HBM
+// rate), 256x256x512 FP32 576 -> 172 us, 64x64x128 FP64 84 -> 34 us.
 constexpr int kDiagZ = 64;
 constexpr int kDiagG = 4;   // planes a group
+constexpr int kDiagBlocks = 592;
+
+// the block's nine values reduced over its threads into v on thread 0 (fixed
+// order): l2, its compensation, max, min, sol, comp., fe, comp., bad cells
+__device__ __forceinline__ void diag_merge(double* v, const double* o)
+{
+    KSum a{v[0], v[1]}; a.merge(o[0], o[1]); v[0] = a.s; v[1] = a.c;
+    v[2] = nan_max(v[2], o[2]); v[3] = nan_min(v[3], o[3]);
+    KSum b{v[4], v[5]}; b.merge(o[4], o[5]); v[4] = b.s; v[5] = b.c;
+    KSum e{v[6], v[7]}; e.merge(o[6], o[7]); v[6] = e.s; v[7] = e.c;
+    v[8] += o[8];
+}
+__device__ __forceinline__ void diag_block_reduce(double* v, double (*sh)[9])
+{
+    for (int off = 16; off > 0; off >>= 1) {
+        double o[9];
+        for (int q = 0; q < 9; ++q) o[q] = __shfl_down_sync(0xffffffffu, v[q], off);
+        diag_merge(v, o);
+    }
+    const int w = threadIdx.x >> 5;
+    __syncthreads();
+    if ((threadIdx.x & 31) == 0)
+        for (int q = 0; q < 9; ++q) sh[w][q] = v[q];
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int ww = 1; ww < (int)(blockDim.x >> 5); ++ww) diag_merge(v, sh[ww]);
+}
+
 template <typename T>
 __global__ void __launch_bounds__(256, 4) k_diag(DomainDesc d, const T* __restrict__ pn, const T* __restrict__ cn,
-                                                 const T* __restrict__ tw, const T* __restrict__ dw,
-                                                 double* __restrict__ part)
+                                                 const T* __restrict__ tw, const T* __restrict__ dw, int zlen,
+                                                 double* __restrict__ part, double* __restrict__ out)
 {
     KSum l2{0, 0}, sol{0, 0}, fe{0, 0};
-    double mx = -DBL_MAX, mn = DBL_MAX, bad = 0.0;
+    double mx = -DBL_MAX, mn = DBL_MAX;
+    int bad = 0;
+    bool nan_phi = false;
     const int nx = d.nx, ny = d.ny, nz = d.nz;
     const long long px = d.px, pl = d.plane;
-    const double dx = d.dx, dy = d.dy, dz = d.dz, w0 = d.W0, hx = d.hx, hy = d.hy, hz = d.hz;
-    const double hE2 = __dmul_rn(__dmul_rn(0.5, d.E0), d.E0);
-    __shared__ double sp[2][kDiagG][8][32];   // the group's phase planes, double-buffered by group parity
+    const double hE2 = 0.5 * d.E0 * d.E0, vol = d.dx * d.dy * d.dz;
+    const double kx = hE2 * d.hx * d.hx, ky = hE2 * d.hy * d.hy, kz = hE2 * d.hz * d.hz;
+    constexpr int W = 34, H = 10;
+    __shared__ double sp[2][kDiagG][H * W];   // the group's phase planes and their ring, double-buffered by group parity
     const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-    const int ntx = (nx + 31) >> 5, nty = (ny + 7) >> 3, ntz = (nz + kDiagZ - 1) / kDiagZ;
+    const int ntx = (nx + 31) >> 5, nty = (ny + 7) >> 3, ntz = (nz + zlen - 1) / zlen;
     const long long ntiles = (long long)ntx * nty * ntz;
-    long long plk[kDiagG + 1];   // k planes, in elements
-#pragma unroll
-    for (int k = 0; k <= kDiagG; ++k) plk[k] = (long long)k * pl;
+    const int me = (ty + 1) * W + tx + 1;
+    // the first 80 threads fetch the tile's ring (its corners are not read)
+    const int h = threadIdx.x;
+    const bool ringer = h < 80;
+    const int hx = h < 64 ? (h & 31) : (h < 72 ? -1 : 32), hy = h < 32 ? -1 : h < 64 ? 8 : (h & 7);
+    const int hs = (hy + 1) * W + hx + 1;
     int g = 0;   // group parity across the whole walk
     for (long long t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const int bx = (int)(t % ntx);
@@ -148,124 +194,101 @@ __global__ void __launch_bounds__(256, 4) k_diag(DomainDesc d, const T* __restri
         const int x = bx * 32 + tx, y = by * 8 + ty;
         const bool own = x < nx && y < ny;
         const bool xy_in = x > 0 && x < nx - 1 && y > 0 && y < ny - 1;
-        const int z0 = bz * kDiagZ, z1 = min(z0 + kDiagZ, nz);
-        const long long col = own ? (long long)x + (long long)y * px : 0;
+        const int z0 = bz * zlen, z1 = min(z0 + zlen, nz);
+        // threads outside the domain repeat its last column: their loads and
+        // extremes are harmless, their sums are dropped
+        const uint32_t col = (uint32_t)min(x, nx - 1) + (uint32_t)min(y, ny - 1) * (uint32_t)px;
+        const uint32_t hcol = (uint32_t)max(min(bx * 32 + hx, nx - 1), 0) +
+                              (uint32_t)max(min(by * 8 + hy, ny - 1), 0) * (uint32_t)px;
         // phase field of this column at planes z-1 (pprev) and z (pcur) of the group's first plane z
-        double pprev = (own && z0 > 0) ? (double)pn[col + (long long)(z0 - 1) * pl] : 0.0;
-        double pcur = own ? (double)pn[col + (long long)z0 * pl] : 0.0;
-        double s_l2 = 0.0, s_sol = 0.0, s_fe = 0.0;   // this column's sums over the chunk
+        double pprev = (double)(pn + (long long)max(z0 - 1, 0) * pl)[col];
+        double pcur = (double)(pn + (long long)z0 * pl)[col];
+        double s_l2 = 0.0, s_sol = 0.0, s_x = 0.0, s_y = 0.0, s_z = 0.0, s_w = 0.0;   // this column's sums
+        int s_bad = 0;
         for (int zb = z0; zb < z1; zb += kDiagG, g ^= 1) {
             const int ng = min(kDiagG, z1 - zb);          // planes in this group (uniform)
-            const long long ib = col + (long long)zb * pl;
-            double pnx[kDiagG], cv[kDiagG], tv[kDiagG], dv[kDiagG];   // phi of plane zb+k+1; c, T, DPP of zb+k
+            // phi of plane zb+k+1; c, T, DPP and the ring of zb+k.  Planes are
+            // clamped to the domain and no load stands under a condition: a
+            // conditional load is waited for inside its branch when a
+            // conversion follows it
+            T pnx[kDiagG], cv[kDiagG], tv[kDiagG], dv[kDiagG], rv[kDiagG];
 #pragma unroll
             for (int k = 0; k < kDiagG; ++k) {
-                const bool in = own && k < ng;
-                pnx[k] = (in && zb + k + 1 < nz) ? (double)pn[ib + plk[k + 1]] : 0.0;
-                cv[k] = in ? (double)cn[ib + plk[k]] : 0.0;
-                tv[k] = (in && tw) ? (double)tw[ib + plk[k]] : 0.0;
-                dv[k] = (in && dw) ? (double)dw[ib + plk[k]] : 0.0;
+                const long long zo = (long long)min(zb + k, nz - 1) * pl;
+                pnx[k] = (pn + (long long)min(zb + k + 1, nz - 1) * pl)[col];
+                cv[k] = (cn + zo)[col];
+                tv[k] = (tw + zo)[col];
+                dv[k] = (dw + zo)[col];
+                rv[k] = (pn + zo)[hcol];
             }
+            double p[kDiagG + 2];   // phi of planes zb-1 .. zb+kDiagG
+            p[0] = pprev;
+            p[1] = pcur;
 #pragma unroll
-            for (int k = 0; k < kDiagG; ++k) sp[g][k][ty][tx] = (k == 0) ? pcur : pnx[k - 1];
+            for (int k = 0; k < kDiagG; ++k) p[k + 2] = (double)pnx[k];
+#pragma unroll
+            for (int k = 0; k < kDiagG; ++k) {
+                sp[g][k][me] = p[k + 1];
+                if (ringer) sp[g][k][hs] = (double)rv[k];
+            }
             __syncthreads();
 #pragma unroll
             for (int k = 0; k < kDiagG; ++k) {
-                if (k >= ng || !own) continue;
+                if (k >= ng) continue;
                 const int z = zb + k;
-                const double phi = (k == 0) ? pcur : pnx[k - 1];
-                const double pm = (k == 0) ? pprev : ((k == 1) ? pcur : pnx[k - 2]);
-                const double pp = pnx[k];
-                s_l2 += phi * phi;
-                mx = nan_max(mx, phi);
-                mn = nan_min(mn, phi);
-                s_sol += cv[k];
-                bool fin = isfinite(phi) && isfinite(cv[k]);
-                if (tw) fin = fin && isfinite(tv[k]);
-                if (dw) fin = fin && isfinite(dv[k]);
-                if (!fin) bad += 1.0;
-                const double w_term = __dmul_rn(__dmul_rn(__dmul_rn(__dmul_rn(w0, phi), phi), 1.0 - phi), 1.0 - phi);
-                double grad2 = 0.0;
-                if (xy_in && z > 0 && z < nz - 1) {
-                    const long long id = ib + plk[k];
-                    const double xp = tx < 31 ? sp[g][k][ty][tx + 1] : (double)pn[id + 1];
-                    const double xm = tx > 0 ? sp[g][k][ty][tx - 1] : (double)pn[id - 1];
-                    const double yp = ty < 7 ? sp[g][k][ty + 1][tx] : (double)pn[id + px];
-                    const double ym = ty > 0 ? sp[g][k][ty - 1][tx] : (double)pn[id - px];
-                    const double gx = __dmul_rn(xp - xm, hx);
-                    const double gy = __dmul_rn(yp - ym, hy);
-                    const double gz = __dmul_rn(pp - pm, hz);
-                    grad2 = __dadd_rn(__dadd_rn(__dmul_rn(gx, gx), __dmul_rn(gy, gy)), __dmul_rn(gz, gz));
+                const double phi = p[k + 1];
+                s_l2 = __fma_rn(phi, phi, s_l2);
+                mx = phi > mx ? phi : mx;
+                mn = phi < mn ? phi : mn;
+                s_sol += (double)cv[k];
+                if (not_finite(phi) || not_finite(cv[k]) || not_finite(tv[k]) || not_finite(dv[k])) {
+                    ++s_bad;
+                    nan_phi = nan_phi || phi != phi;
                 }
-                const double e = __dadd_rn(__dmul_rn(hE2, grad2), w_term);
-                s_fe += __dmul_rn(__dmul_rn(__dmul_rn(e, dx), dy), dz);
+                const double w = phi * (1.0 - phi);
+                s_w = __fma_rn(w, w, s_w);
+                if (z > 0 && z < nz - 1) {
+                    const double* const q = &sp[g][k][me];
+                    const double gx = q[1] - q[-1], gy = q[W] - q[-W], gz = p[k + 2] - p[k];
+                    s_x = __fma_rn(gx, gx, s_x);
+                    s_y = __fma_rn(gy, gy, s_y);
+                    s_z = __fma_rn(gz, gz, s_z);
+                }
             }
-            if (ng == kDiagG) {   // the next group's planes z-1 and z (a short group ends the chunk)
-                pprev = pnx[kDiagG - 2];
-                pcur = pnx[kDiagG - 1];
-            }
+            pprev = p[kDiagG];   // the next group's planes z-1 and z (a short group ends the chunk)
+            pcur = p[kDiagG + 1];
         }
-        l2.add(s_l2);
-        sol.add(s_sol);
-        fe.add(s_fe);
+        if (own) {
+            const double e = xy_in ? __fma_rn(kx, s_x, __fma_rn(ky, s_y, kz * s_z)) : 0.0;
+            l2.add(s_l2);
+            sol.add(s_sol);
+            fe.add(vol * __fma_rn(d.W0, s_w, e));
+            bad += s_bad;
+        }
     }
+    if (nan_phi) mx = mn = __longlong_as_double(0x7ff8000000000000ll);
     __shared__ double sh[8][9];
-    double v[9] = {l2.s, l2.c, mx, mn, sol.s, sol.c, fe.s, fe.c, bad};
-    // warp reduction (fixed order, deterministic for a fixed launch shape)
-    for (int off = 16; off > 0; off >>= 1) {
-        double o[9];
-        for (int q = 0; q < 9; ++q) o[q] = __shfl_down_sync(0xffffffffu, v[q], off);
-        KSum a{v[0], v[1]}; a.merge(o[0], o[1]); v[0] = a.s; v[1] = a.c;
-        v[2] = nan_max(v[2], o[2]); v[3] = nan_min(v[3], o[3]);
-        KSum b{v[4], v[5]}; b.merge(o[4], o[5]); v[4] = b.s; v[5] = b.c;
-        KSum e{v[6], v[7]}; e.merge(o[6], o[7]); v[6] = e.s; v[7] = e.c;
-        v[8] += o[8];
-    }
-    int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-    if (l == 0)
-        for (int q = 0; q < 9; ++q) sh[w][q] = v[q];
-    __syncthreads();
+    __shared__ bool last;
+    double v[9] = {l2.s, l2.c, mx, mn, sol.s, sol.c, fe.s, fe.c, (double)bad};
+    diag_block_reduce(v, sh);
+    unsigned* const done = (unsigned*)(out + 7);   // blocks that have written their partials; 0 between launches
     if (threadIdx.x == 0) {
-        int nw = blockDim.x >> 5;
-        for (int q = 0; q < 9; ++q) v[q] = sh[0][q];
-        for (int ww = 1; ww < nw; ++ww) {
-            KSum a{v[0], v[1]}; a.merge(sh[ww][0], sh[ww][1]); v[0] = a.s; v[1] = a.c;
-            v[2] = nan_max(v[2], sh[ww][2]); v[3] = nan_min(v[3], sh[ww][3]);
-            KSum b{v[4], v[5]}; b.merge(sh[ww][4], sh[ww][5]); v[4] = b.s; v[5] = b.c;
-            KSum e{v[6], v[7]}; e.merge(sh[ww][6], sh[ww][7]); v[6] = e.s; v[7] = e.c;
-            v[8] += sh[ww][8];
-        }
         for (int q = 0; q < 9; ++q) part[(long long)blockIdx.x * kDiagRow + q] = v[q];
+        __threadfence();
+        last = atomicAdd(done, 1u) == gridDim.x - 1;
     }
-}
-
-// One warp merges the per-block partials: lane l takes blocks l, l + 32, ...,
-// then the lanes merge in a fixed shuffle order (deterministic).
-template <typename T>  // templated only so each precision unit owns its copy
-__global__ void k_diag_final(const double* __restrict__ part, int nblk, double* __restrict__ out)
-{
-    if (blockIdx.x != 0 || threadIdx.x >= 32) return;
-    KSum l2{0, 0}, sol{0, 0}, fe{0, 0};
-    double mx = -DBL_MAX, mn = DBL_MAX, bad = 0.0;
-    for (int b = (int)threadIdx.x; b < nblk; b += 32) {
-        const double* p = part + (long long)b * kDiagRow;
-        l2.merge(p[0], p[1]);
-        mx = nan_max(mx, p[2]);
-        mn = nan_min(mn, p[3]);
-        sol.merge(p[4], p[5]);
-        fe.merge(p[6], p[7]);
-        bad += p[8];
-    }
-    double v[9] = {l2.s, l2.c, mx, mn, sol.s, sol.c, fe.s, fe.c, bad};
-    for (int off = 16; off > 0; off >>= 1) {
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int q = 0; q < 9; ++q) v[q] = 0.0;
+    v[2] = -DBL_MAX;
+    v[3] = DBL_MAX;
+    for (int b = (int)threadIdx.x; b < (int)gridDim.x; b += (int)blockDim.x) {
         double o[9];
-        for (int q = 0; q < 9; ++q) o[q] = __shfl_down_sync(0xffffffffu, v[q], off);
-        KSum a{v[0], v[1]}; a.merge(o[0], o[1]); v[0] = a.s; v[1] = a.c;
-        v[2] = nan_max(v[2], o[2]); v[3] = nan_min(v[3], o[3]);
-        KSum b{v[4], v[5]}; b.merge(o[4], o[5]); v[4] = b.s; v[5] = b.c;
-        KSum e{v[6], v[7]}; e.merge(o[6], o[7]); v[6] = e.s; v[7] = e.c;
-        v[8] += o[8];
+        for (int q = 0; q < 9; ++q) o[q] = __ldcg(part + (long long)b * kDiagRow + q);
+        diag_merge(v, o);
     }
+    diag_block_reduce(v, sh);
     if (threadIdx.x == 0) {
         out[0] = sqrt(v[0] + v[1]);
         out[1] = v[2];
@@ -273,6 +296,7 @@ __global__ void k_diag_final(const double* __restrict__ part, int nblk, double* 
         out[3] = v[4] + v[5];
         out[4] = v[6] + v[7];
         out[5] = v[8];   // cells with a non-finite phi, c, T or DPP (the watchdog)
+        *done = 0u;
     }
 }
 
@@ -326,12 +350,22 @@ cudaError_t launch_copy_inner(const DomainDesc& d, const void* src, void* dst, c
     return cudaGetLastError();
 }
 
+// part: kDiagBlocks rows; out: 8 doubles, the last one zero before the first call
 template <typename T>
 cudaError_t launch_diag(const DomainDesc& d, const void* phi, const void* c, const void* Tw, const void* dppw,
-                        double* part, int nblk, double* out, cudaStream_t st)
+                        double* part, double* out, cudaStream_t st)
 {
-    k_diag<T><<<nblk, 256, 0, st>>>(d, (const T*)phi, (const T*)c, (const T*)Tw, (const T*)dppw, part);
-    k_diag_final<T><<<1, 32, 0, st>>>(part, nblk, out);
+    // chunks of whole groups, short enough for a small domain's tiles to fill
+    // the grid, at most kDiagZ planes
+    const long long cols = (long long)((d.nx + 31) / 32) * ((d.ny + 7) / 8);
+    const long long want = (kDiagBlocks + cols - 1) / cols;   // chunks a column
+    long long zlen = ((d.nz + want - 1) / want + kDiagG - 1) / kDiagG * kDiagG;
+    zlen = zlen < kDiagZ ? zlen : kDiagZ;
+    const long long tiles = cols * ((d.nz + zlen - 1) / zlen);
+    const int nblk = (int)(tiles < kDiagBlocks ? tiles : kDiagBlocks);
+    // a field the watchdog does not look at is replaced by c, which it does
+    k_diag<T><<<nblk, 256, 0, st>>>(d, (const T*)phi, (const T*)c, (const T*)(Tw ? Tw : c),
+                                    (const T*)(dppw ? dppw : c), (int)zlen, part, out);
     return cudaGetLastError();
 }
 

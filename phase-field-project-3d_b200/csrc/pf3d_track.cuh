@@ -9,8 +9,8 @@
 //
 // One pass over phi: each CTA reduces a band of rows of one plane to the
 // plane's maximum (an order-preserving 64-bit key, so atomicMax is exact and
-// order independent) and its count of solid cells (integer, exact); a one-thread
-// kernel then scans the plane maxima from the top.  The result equals the same
+// order independent) and its count of solid cells (integer, exact); one warp
+// then scans the plane maxima from the top.  The result equals the same
 // metric evaluated on the downloaded field bit for bit.
 #pragma once
 #include "pf3d_launch.h"
@@ -79,10 +79,15 @@ template <typename T>
 __global__ void k_track_final(int nz, long long cells, const unsigned long long* __restrict__ pmax,
                               const unsigned long long* __restrict__ count, double* __restrict__ out)
 {
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
+    // one warp, 32 planes at a time from the top (one plane at a time is a
+    // chain of dependent reads: 150 us for 300 planes of melt)
     int k = -1;
-    for (int z = nz - 1; z >= 0; --z)
-        if (track_unkey(pmax[z]) >= 0.5) { k = z; break; }
+    for (int zt = nz - 1; zt >= 0 && k < 0; zt -= 32) {
+        const int z = zt - (int)threadIdx.x;
+        const unsigned hit = __ballot_sync(0xffffffffu, z >= 0 && track_unkey(pmax[z >= 0 ? z : 0]) >= 0.5);
+        if (hit) k = zt - (__ffs(hit) - 1);
+    }
+    if (threadIdx.x != 0) return;
     double tip = 0.0;
     if (k >= 0) {
         if (k + 1 >= nz) {
