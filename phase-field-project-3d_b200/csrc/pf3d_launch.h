@@ -8,6 +8,30 @@
 
 namespace pf3d {
 
+// Launches a kernel that calls pdl_wait() before it touches global memory, so
+// that its blocks may be set up while the stream's previous kernel drains: a
+// step of a small domain is a chain of 10 us kernels, and the set-up of each
+// showed as a gap.  The march passes release in their last plane (36x32x48 FP64
+// 22.6 -> 19.1 us a step, 64x64x128 FP64 51.3 -> 46.8 us, large domains 0.5 %
+// faster); released at their start, the early blocks crowd onto the SMs that
+// finish first and larger domains lose 1 to 5 %.  Not for the Karma passes,
+// whose blocks differ by the crystal they hold: 200^3 FP64 328 -> 350 us.
+template <typename... P, typename... A>
+inline cudaError_t launch_pdl(void (*kern)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... a)
+{
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cudaLaunchAttribute at = {};
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(a)...);
+}
+
 // Device pointers of one domain.  "old"/"new" follow the reference names.
 struct Fields {
     void* phi_old;

@@ -388,6 +388,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
         if (SOL) load_c(z + 2, c_in + zoff + 2 * pl, c2, cr2, IN || zdom(z + 2));
         else load_c(z + 1, c_in + zoff + pl, c1, cr1, IN || zdom(z + 1));
 
+        if (!IN && z == ze - 1) pdl_release();   // the last plane is never an IN one
         // A: plane z+2 has landed
         if (IN || z + 2 <= zlast) bad |= !wait_plane(sq);
         // B, C: nodes and solute points of plane z+1
@@ -602,7 +603,9 @@ __global__ void __launch_bounds__(32 * TY / L, (MarchOcc<S, L, SMOOTH, PHASE, FA
 {
     extern __shared__ __align__(128) unsigned char smem_raw[];
     unsigned char* smem = align128(smem_raw);
+    if (threadIdx.x == 0 && threadIdx.y == 0) prefetch_tensormap(&tm);
     march_init_barriers<MarchLayout<S, TY, SOL, PHASE, FAST>>(smem);
+    pdl_wait();
     uint32_t par = 0;
     if (!march_any<S, L, TY, HEAT, DPPW, SOL, SMOOTH, sizeof(S) == 8, PHASE, FAST, HQ>(
             d, c, cv, &tm, c_in, phi_out, dpp, c_out, T_old, T_new, zchunk, blockIdx.x, blockIdx.y, blockIdx.z, smem,
@@ -739,9 +742,8 @@ cudaError_t launch_march_t(const CUtensorMap& tm, const DomainDesc& d, const Ste
     kc.load(d, s);
     const auto kv = kc_lanes<S, L>(kc);
     dim3 grid((d.nx + 31) / 32, (d.ny + TY - 1) / TY, (d.nz + zchunk - 1) / zchunk);
-    kern<<<grid, dim3(32, TY / L), LY::ALLOC, st>>>(tm, d, kc, kv, (const S*)c_in, (S*)phi_out, (S*)dpp, (S*)c_out,
-                                                     (const S*)T_old, (S*)T_new, zchunk, err);
-    return cudaGetLastError();
+    return launch_pdl(kern, grid, dim3(32, TY / L), LY::ALLOC, st, tm, d, kc, kv, (const S*)c_in, (S*)phi_out,
+                      (S*)dpp, (S*)c_out, (const S*)T_old, (S*)T_new, zchunk, err);
 }
 
 // the passes of a step (32 x 8 tiles).  lanes: cells per thread (1 or 2); the
