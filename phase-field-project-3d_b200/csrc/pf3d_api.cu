@@ -107,8 +107,9 @@ static int cuda_check(pf_ctx* c, cudaError_t e, const char* what)
 
 static inline bool is64(const pf_ctx* c) { return c->prec == PF_FP64; }
 
-// CTAs of the march passes an SM holds, for the chunk rule: FP64 with the
-// smooth noise 2, otherwise FP64 and one FP32 cell a thread 3, FP32 pairs 6
+// CTAs of the march passes an SM holds, for the chunk rule: the FP64 reference
+// form's sweep and one-sweep step 2, otherwise FP64 and one FP32 cell a thread
+// 3, FP32 pairs 6
 static const int kMarchOcc[3] = {2, 3, 6};
 
 extern "C" {
@@ -696,7 +697,7 @@ static int one_step(pf_ctx* ctx)
         // TMA-staged passes: two cells per thread unless PF_OPT_PAIRED says
         // otherwise (default: FP32 only) or the deck draws the smooth noise
         const int lanes = ((ctx->paired == 2 || (ctx->paired == 1 && !is64(ctx))) && p.ruido_tipo != 2) ? 2 : 1;
-        const int occ_q = (is64(ctx) && p.ruido_tipo == 2) ? 0 : (lanes == 2 && !is64(ctx)) ? 2 : 1;
+        const int occ_q = (lanes == 2 && !is64(ctx)) ? 2 : (is64(ctx) && nsw == 1) ? 0 : 1;
         const int zchunk = ctx->zchunk_set ? ctx->zchunk : ctx->zfill[occ_q];
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         f.phi_mid = B;

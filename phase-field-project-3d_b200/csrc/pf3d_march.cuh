@@ -363,6 +363,19 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
     if (PHASE && zin(zb - 1)) node_plane(nm, phi_at((zb + 4) % 6), phi_at((zb + 5) % 6), phi_at(zb % 6));
     if (PHASE && zin(zb)) node_plane(n0, phi_at((zb + 5) % 6), phi_at(zb % 6), phi_at((zb + 1) % 6));
 
+    // the smooth noise's lattice layers below and above the plane, blended at the
+    // own columns: they change every six planes, and the upper one becomes the
+    // lower, so a cell costs a blend of two numbers and two thirds of a hash
+    // where it took eight hashes (97x131x201 FP64, one
+    // sweep: 211 -> 177 us a step)
+    double slo[L], shi[L];
+    const bool smooth = SMOOTH && c.rt == 2;
+    auto smooth_layer = [&](int l, int k0) { return ruido_layer64(x0 + tx + 1, y0 + ty + l * TR + 1, k0, c.it); };
+#pragma unroll
+    for (int l = 0; l < L; ++l) {
+        slo[l] = smooth ? smooth_layer(l, (zb + 1) / 6) : 0.0;
+        shi[l] = smooth ? smooth_layer(l, (zb + 1) / 6 + 1) : 0.0;
+    }
     uint64_t hin[L];   // noise hash input of the own cells, carried along z (k = z + 1)
 #pragma unroll
     for (int l = 0; l < L; ++l)
@@ -418,8 +431,15 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
             } else if constexpr (ran_mode == 2) {
                 ran[l] = dcur[l];
             } else if constexpr (SMOOTH) {
-                ran[l] = (S)((c.rt == 2) ? phase_ran(2, x0 + tx + 1, y0 + ty + l * TR + 1, z + 1, c.it)
-                                         : __double2float_rn(ran64(hash63_mix(hin[l]))));
+                if (smooth) {
+                    if ((z + 1) % 6 == 0 && z > zb) {
+                        slo[l] = shi[l];
+                        shi[l] = smooth_layer(l, (z + 1) / 6 + 1);
+                    }
+                    ran[l] = (S)__double2float_rn(ruido_blend64(slo[l], shi[l], z + 1));
+                } else {
+                    ran[l] = (S)__double2float_rn(ran64(hash63_mix(hin[l])));
+                }
             } else {
                 ran[l] = (S)__double2float_rn(ran64(hash63_mix(hin[l])));
             }
@@ -585,17 +605,18 @@ __device__ __forceinline__ bool march_any(const DomainDesc& d, const KC<S>& c, c
 }
 
 // resident CTAs per SM the register budget is sized for (shared memory
-// allows no more): FP64 3 (80 registers a thread), or 2 for a pass that may
-// draw the smooth noise (its trilinear blend of eight hashes) and for the
-// reference form of the sweep; FP32 pairs 6, FP32 single cells 3
-template <typename S, int L, bool SMOOTH, bool PHASE = true, bool FAST = true>
+// allows no more): FP64 3 (80 registers a thread), or 2 for the reference form
+// of the sweep and for the whole step of one sweep in one pass (300x300x200:
+// 755 us a step with 3 and its spills, 683 with 2); FP32 pairs 6, FP32 single
+// cells 3
+template <typename S, int L, bool PHASE = true, bool FAST = true, bool ONE = false>
 struct MarchOcc {
-    static constexpr int v = (sizeof(S) == 8) ? ((SMOOTH || (PHASE && !FAST)) ? 2 : 3) : (L == 2 ? 6 : 3);
+    static constexpr int v = (sizeof(S) == 8) ? (((PHASE && !FAST) || ONE) ? 2 : 3) : (L == 2 ? 6 : 3);
 };
 
 // single domain: one CTA per tile; the phase field comes through `tm`
 template <typename S, int L, int TY, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool PHASE, bool FAST, int HQ>
-__global__ void __launch_bounds__(32 * TY / L, (MarchOcc<S, L, SMOOTH, PHASE, FAST>::v))
+__global__ void __launch_bounds__(32 * TY / L, (MarchOcc<S, L, PHASE, FAST, HEAT && SOL>::v))
     k_march(const __grid_constant__ CUtensorMap tm, DomainDesc d, const KC<S> c,
             const KC<typename Lanes<S, L>::V> cv, const S* __restrict__ c_in, S* __restrict__ phi_out,
             S* __restrict__ dpp, S* __restrict__ c_out, const S* __restrict__ T_old, S* __restrict__ T_new,
@@ -624,7 +645,7 @@ __global__ void __launch_bounds__(32 * TY / L, (MarchOcc<S, L, SMOOTH, PHASE, FA
 // z-chunks, small domains at the end of the largest-first list) keep
 // working while others finish long ones.
 template <typename S, int L, int TY, int PASS, bool ONE_SWEEP, bool SMOOTH>
-__global__ void __launch_bounds__(32 * TY / L, (MarchOcc<S, L, SMOOTH>::v))
+__global__ void __launch_bounds__(32 * TY / L, (MarchOcc<S, L, true, true, ONE_SWEEP>::v))
     k_march_batch(const BatchDomain* __restrict__ doms, const CUtensorMap* __restrict__ tmaps,
                   const BatchStep* __restrict__ steps, const BatchItem* __restrict__ items,
                   const int* __restrict__ head, int* __restrict__ ctr, int* __restrict__ err)
@@ -757,7 +778,10 @@ cudaError_t launch_march_first(const CUtensorMap& tm, const DomainDesc& d, const
                                                               SO ? f.c_new : nullptr, f.T_old, f.T_new, zchunk, \
                                                               err, st)
 #define PF3D_MQ(L, SO) (d.hq ? PF3D_MF(L, SO, false, 1) : PF3D_MF(L, SO, false, 0))
-    if (d.rt == 2) return with_solute ? PF3D_MF(1, true, true, 2) : PF3D_MF(1, false, true, 2);
+    if (d.rt == 2) {
+        if (with_solute) return d.hq ? PF3D_MF(1, true, true, 1) : PF3D_MF(1, true, true, 0);
+        return d.hq ? PF3D_MF(1, false, true, 1) : PF3D_MF(1, false, true, 0);
+    }
     if (with_solute) return lanes == 2 ? PF3D_MQ(2, true) : PF3D_MQ(1, true);
     return lanes == 2 ? PF3D_MQ(2, false) : PF3D_MQ(1, false);
 #undef PF3D_MQ
