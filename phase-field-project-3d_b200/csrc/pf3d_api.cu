@@ -699,12 +699,13 @@ static int one_step(pf_ctx* ctx)
         const int lanes = ((ctx->paired == 2 || (ctx->paired == 1 && !is64(ctx))) && p.ruido_tipo != 2) ? 2 : 1;
         const int occ_q = (lanes == 2 && !is64(ctx)) ? 2 : (is64(ctx) && nsw == 1) ? 0 : 1;
         const int zchunk = ctx->zchunk_set ? ctx->zchunk : ctx->zfill[occ_q];
+        const bool flat = nsw == 2 && ctx->g.nz >= kFlatDepth && (zchunk >= kFlatChunk || zchunk == 0);
         cudaEvent_t e0 = nullptr, e1 = nullptr;
         f.phi_mid = B;
         if (ctx->ktiming) { e0 = new_event(); e1 = new_event(); cudaEventRecord(e0, ctx->stream); }
-        CK(is64(ctx) ? launch_march_first<double>(tm_of(ctx, A), ctx->dd, s, f, nsw == 1, lanes, zchunk,
+        CK(is64(ctx) ? launch_march_first<double>(tm_of(ctx, A), ctx->dd, s, f, nsw == 1, lanes, flat, zchunk,
                                                   ctx->d_status, ctx->stream)
-                     : launch_march_first<float>(tm_of(ctx, A), ctx->dd, s, f, nsw == 1, lanes, zchunk,
+                     : launch_march_first<float>(tm_of(ctx, A), ctx->dd, s, f, nsw == 1, lanes, flat, zchunk,
                                                  ctx->d_status, ctx->stream),
            nsw == 1 ? "march step (single sweep)" : "march heat + sweep 1");
         if (ctx->ktiming) { cudaEventRecord(e1, ctx->stream); ctx->ev_first.push_back({e0, e1}); }
@@ -723,9 +724,9 @@ static int one_step(pf_ctx* ctx)
             f2.phi_mid = cur;
             f2.phi_new = oth;
             if (ctx->ktiming) { e0 = new_event(); e1 = new_event(); cudaEventRecord(e0, ctx->stream); }
-            CK(is64(ctx) ? launch_march_last<double>(tm_of(ctx, cur), ctx->dd, s, f2, lanes, zchunk,
+            CK(is64(ctx) ? launch_march_last<double>(tm_of(ctx, cur), ctx->dd, s, f2, lanes, flat, zchunk,
                                                      ctx->d_status, ctx->stream)
-                         : launch_march_last<float>(tm_of(ctx, cur), ctx->dd, s, f2, lanes, zchunk,
+                         : launch_march_last<float>(tm_of(ctx, cur), ctx->dd, s, f2, lanes, flat, zchunk,
                                                     ctx->d_status, ctx->stream),
                "march last sweep + solute");
             if (ctx->ktiming) { cudaEventRecord(e1, ctx->stream); ctx->ev_last.push_back({e0, e1}); }

@@ -100,11 +100,13 @@ template <typename T> cudaError_t launch_fused_batch_pair(const BatchDomain* dom
 // phase field through the tensor map `tm`, `lanes` cells per thread (1 or 2);
 // a plane load that does not arrive sets *err.  Same outputs, bit for bit, as launch_fused_first / _last.
 template <typename S> cudaError_t launch_march_first(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s,
-                                                     const Fields& f, bool with_solute, int lanes, int zchunk,
-                                                     int* err, cudaStream_t st);
+                                                     const Fields& f, bool with_solute, int lanes, bool flat,
+                                                     int zchunk, int* err, cudaStream_t st);
 template <typename S> cudaError_t launch_march_last(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s,
-                                                    const Fields& f, int lanes, int zchunk, int* err,
+                                                    const Fields& f, int lanes, bool flat, int zchunk, int* err,
                                                     cudaStream_t st);
+// planes of the domain and of a chunk from which `flat` serves (launch_march_first)
+constexpr int kFlatDepth = 448, kFlatChunk = 24;
 // one subroutine alone (FP64: reference form): a phase sweep (dpp may be null)
 // and the solute update
 template <typename S> cudaError_t launch_march_sweep(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s,

@@ -77,7 +77,8 @@ struct MarchLayout {
     static constexpr int PHI_BYTES = TW * PH * ES;
     static_assert(PHI_BYTES % 128 == 0, "TMA destinations are 128-byte aligned");
     static constexpr int BAR_OFF = NPHI * PHI_BYTES;
-    static constexpr int NODE_OFF = (BAR_OFF + NPHI * 8 + 127) / 128 * 128;
+    static constexpr int BAD_OFF = BAR_OFF + NPHI * 8;   // set by a thread whose plane load did not arrive
+    static constexpr int NODE_OFF = (BAD_OFF + 4 + 127) / 128 * 128;
     // arrays of a slot: eps^2, exy, eyz, ezx; Gamma bracket, mu (reference
     // form 1/GAMMA, mu, 1/GAMMA of the solid)
     static constexpr int Q_SOL = PHASE ? 4 : 0;
@@ -125,6 +126,7 @@ __device__ __forceinline__ void march_init_barriers(unsigned char* smem)
     if (threadIdx.x == 0 && threadIdx.y == 0) {
         const uint32_t b0 = smem_u32(smem + LY::BAR_OFF);
         for (int s = 0; s < LY::NPHI; ++s) mbar_init(b0 + 8 * s, 1);
+        *reinterpret_cast<int*>(smem + LY::BAD_OFF) = 0;
         fence_mbar_init();
     }
     __syncthreads();
@@ -140,7 +142,9 @@ __device__ __forceinline__ void march_init_barriers(unsigned char* smem)
 // second store (FP64).
 // PHASE = false leaves the phase sweep out (the solute subroutine alone);
 // FAST = false is the reference form of the per-subroutine entry points (FP64,
-// one lane).
+// one lane).  FLAT: planes on which the tile holds nothing but 0 or nothing but
+// 1 (melt beyond the interface's tail, the crystal's interior) leave out what
+// is exactly zero there (two-sweep steps, below).
 //
 // The arithmetic is a third to a half of what a plane executes: the rest is
 // addresses, conditions and moves, and every thread repeats it in every
@@ -157,7 +161,7 @@ __device__ __forceinline__ void march_init_barriers(unsigned char* smem)
 // barriers), the logarithm's coefficients in the constant bank (pass 2 10 %
 // slower), 2 CTAs an SM with 128 registers (4 % slower).
 template <typename S, int L, int TY, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool SPLIT, bool PHASE, bool FAST,
-          int HQ, bool INT>
+          int HQ, bool FLAT, bool INT>
 __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, const KC<typename Lanes<S, L>::V>& cv,
                                            const CUtensorMap* tm, const S* __restrict__ c_in,
                                            S* __restrict__ phi_out, S* __restrict__ dpp, S* __restrict__ c_out,
@@ -200,7 +204,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
     const bool ring_s = SOL && tid >= NT - NRING;       // ring solute points
     uint32_t col[L], rcol[L];      // element offsets in the plane: own cells, ring points
     uint32_t rphi[L], rnode[L];    // bytes from the thread's own position (lane 0) to its ring items
-    bool own[L], xyin[L], rin[L];
+    bool own[L], xyin[L], rin[L], rdom[L];
     {
         int r = ring ? tid : (ring_s ? tid - (NT - NRING) : 0), rx[L], ry[L];
         if (L == 1) {
@@ -222,6 +226,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
             const int x = x0 + tx, y = y0 + ty + l * TR, gx = x0 - 1 + rx[l], gy = y0 - 1 + ry[l];
             own[l] = INT || (x < nx && y < ny);
             xyin[l] = INT || (x >= 1 && x <= nx - 2 && y >= 1 && y <= ny - 2);
+            rdom[l] = ring && (INT || (gx >= 0 && gx < nx && gy >= 0 && gy < ny));    // its phase value counts
             rin[l] = ring_s && (INT || (gx >= 0 && gx < nx && gy >= 0 && gy < ny));   // its concentration is read
             col[l] = (uint32_t)x + (uint32_t)y * (uint32_t)px;
             rcol[l] = (uint32_t)gx + (uint32_t)gy * (uint32_t)px;
@@ -289,9 +294,25 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
         stn(dst, 2, q.eyz, rg);
         stn(dst, 3, q.ezx, rg);
     };
-    auto node_plane = [&](uint32_t dst, uint32_t m, uint32_t p0, uint32_t pp) {
-        node_one(dst, m, p0, pp, false);
-        if (ring) node_one(dst, m, p0, pp, true);
+    // own_flat / ring_flat: the warp's gradients there are all zero
+    auto node_plane = [&](uint32_t dst, uint32_t m, uint32_t p0, uint32_t pp, bool own_flat, bool ring_flat) {
+        auto zero = [&](bool rg) {
+            const Node<S> q = aniso_flat<S>(c);
+#pragma unroll
+            for (int l = 0; l < L; ++l) {
+                const uint32_t o = na(dst, l, rg);
+                sts(o, q.eps * q.eps);
+                sts(o + NB, (S)0);
+                sts(o + 2 * NB, (S)0);
+                sts(o + 3 * NB, (S)0);
+            }
+        };
+        if (FLAT && own_flat) zero(false);
+        else node_one(dst, m, p0, pp, false);
+        if (ring) {
+            if (FLAT && ring_flat) zero(true);
+            else node_one(dst, m, p0, pp, true);
+        }
     };
     // solute point quantities of a plane into its slot, from its phase plane
     // and the concentration at the own (co) and ring (cr) points
@@ -360,8 +381,8 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
         wait_first();
     }
     load_centre(zb, zo0, zin(zb));
-    if (PHASE && zin(zb - 1)) node_plane(nm, phi_at((zb + 4) % 6), phi_at((zb + 5) % 6), phi_at(zb % 6));
-    if (PHASE && zin(zb)) node_plane(n0, phi_at((zb + 5) % 6), phi_at(zb % 6), phi_at((zb + 1) % 6));
+    if (PHASE && zin(zb - 1)) node_plane(nm, phi_at((zb + 4) % 6), phi_at((zb + 5) % 6), phi_at(zb % 6), false, false);
+    if (PHASE && zin(zb)) node_plane(n0, phi_at((zb + 5) % 6), phi_at(zb % 6), phi_at((zb + 1) % 6), false, false);
 
     // the smooth noise's lattice layers below and above the plane, blended at the
     // own columns: they change every six planes, and the upper one becomes the
@@ -383,6 +404,9 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
     uint32_t am = phi_at((zb + 5) % 6), a0 = phi_at(zb % 6), ap = phi_at((zb + 1) % 6);   // planes z-1, z, z+1
     int sq = (zb + 2) % 6;       // phase slot of plane z+2
     long long zoff = zo0;
+    // what planes z-1, z and z+1 hold all over the tile and its ring (inside the
+    // domain): 1 exactly 0, 2 exactly 1, 0 anything else or not known yet
+    int un = 0, u0 = 0, u1 = 0;
 
     // One plane of the march.  IN: every z-dependent condition of the plane
     // is known true (z in [3, N-4], the planes it reads and the load it
@@ -404,19 +428,69 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
         if (!IN && z == ze - 1) pdl_release();   // the last plane is never an IN one
         // A: plane z+2 has landed
         if (IN || z + 2 <= zlast) bad |= !wait_plane(sq);
+        // whether plane z+2 holds one of the two values all over, and the
+        // concentrations of plane z keep the driving force's logarithm finite
+        // (0 < c < Ke); and whether the warp's nodes of plane z+1 are flat
+        bool mixed = false, own_flat = false, ring_flat = false;
+        int u2 = u1;
+        if constexpr (FLAT) {
+            if (IN || z + 2 <= zlast) {
+                S v;
+                lds(sb + (uint32_t)(sq * LY::PHI_BYTES + 2 * PR + XOFF * ES), v);   // the tile's first cell
+                u2 = is_bits0(v) ? 1 : is_bits1(v) ? 2 : 0;
+                bool od = false, rd = false;   // own cells, ring items that differ from it
+#pragma unroll
+                for (int l = 0; l < L; ++l) {
+                    S a, b;
+                    lds(pa(aq, l, false), a);
+                    lds(pa(aq, l, true), b);
+                    od = od || (own[l] && a != v);
+                    rd = rd || (rdom[l] && b != v);
+                }
+                mixed = u2 == 0 || od || rd;
+                if (u0 != 0 && u0 == u1 && u1 == u2) {   // planes z and z+1 hold it too (CTA-uniform)
+                    own_flat = !__any_sync(0xffffffffu, od);
+                    ring_flat = !__any_sync(0xffffffffu, rd);
+                }
+            }
+#pragma unroll
+            for (int l = 0; l < L; ++l) mixed = mixed || (own[l] && !(co[l] > (S)0 && co[l] < c.Ke));
+        }
         // B, C: nodes and solute points of plane z+1
-        if (PHASE && (IN || zin(z + 1))) node_plane(np, a0, ap, aq);
+        if (PHASE && (IN || zin(z + 1))) node_plane(np, a0, ap, aq, own_flat, ring_flat);
         if (SOL && (IN || z + 1 <= nz - 1)) sol_plane(np, ap, c1, cr1);
-        // D: one barrier orders the plane; everyone learns of a failed load
-        if (__syncthreads_or(bad)) {
-            drain();
-            return false;
+        // D: one barrier orders the plane; everyone learns of a failed load, and
+        // whether the plane is mixed
+        if constexpr (FLAT) {
+            int* const flag = reinterpret_cast<int*>(smem + LY::BAD_OFF);
+            if (bad) *flag = 1;
+            if (__syncthreads_or(bad || mixed)) {
+                if (*(volatile int*)flag) {
+                    drain();
+                    return false;
+                }
+                u2 = 0;
+            }
+        } else {
+            if (__syncthreads_or(bad)) {
+                drain();
+                return false;
+            }
         }
         // E: the load of plane z+4 into the slot plane z-2 has left (read
         // only, by threads that are behind the barrier)
         if (lead && (IN || z + 4 <= zlast)) issue(z + 4, sq + 2 >= 6 ? sq - 4 : sq + 2);
 
-        // F: the cells of plane z
+        // F: the cells of plane z.  Where planes z-1 .. z+2 hold nothing but 0 or
+        // nothing but 1, every difference, g', h' and the noise's
+        // phi^2 (1-phi)^2 are zero and the sweep changes nothing: the cells
+        // keep their value and DPP is zero, the bits the arithmetic gives as
+        // long as its logarithm is finite.  (The noise is not drawn either:
+        // the second sweep multiplies it by the same zero.)
+        const bool flat = FLAT && un != 0 && un == u0 && u0 == u1 && u1 == u2;
+        un = u0;
+        u0 = u1;
+        u1 = u2;
         const bool zi = IN || zin(z);                     // T interior / phase source / solute interior
         const bool zph = IN || (z >= 2 && z <= nz - 3);   // phase interior
         const V PP = ldv(a0, 0, false);
@@ -426,9 +500,9 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
         S ran[L];
 #pragma unroll
         for (int l = 0; l < L; ++l) {
-            if constexpr (!PHASE) {
+            if (!PHASE || flat) {
                 ran[l] = (S)0;
-            } else if constexpr (ran_mode == 2) {
+            } else if (ran_mode == 2) {
                 ran[l] = dcur[l];
             } else if constexpr (SMOOTH) {
                 if (smooth) {
@@ -447,7 +521,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
         }
 
         V ppn = PP;
-        if (PHASE && zph) {
+        if (PHASE && zph && !flat) {
             Nbr<V> nb;
             nb.PP = PP;
             nb.PN = ldv(a0, PR, false); nb.PS = ldv(a0, -PR, false);
@@ -583,24 +657,54 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
     return true;
 }
 
+// Whether a chunk of the tile looks uniform: four cells of its middle column
+// hold 0, or all 1 (the same answer in every thread).  A guess: the copy of
+// the body it selects is right for any plane.
+template <typename S>
+__device__ __forceinline__ bool looks_flat(const DomainDesc& d, const S* phi, int x0, int y0, int zb, int ze)
+{
+    const S* const p = phi + min(x0 + 16, d.nx - 1) + (long long)min(y0 + 4, d.ny - 1) * d.px;
+    const int n = ze - 1 - zb;
+    S v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = p[(long long)(zb + i * n / 3) * d.plane];
+    bool zero = true, one = true;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+        zero = zero && is_bits0(v[i]);
+        one = one && is_bits1(v[i]);
+    }
+    return zero || one;
+}
+
 // The tile in the copy of the body that its position in the domain needs.  The
 // FP32 passes, with twice the CTAs in flight and half the instructions a cell,
 // are short of instruction cache and run the one copy with all its checks
 // (256^3: 668 us a step with interior copies of tiles and planes, 561 without;
 // FP64 340x340x200: 1290 us with, 1405 without).
+// FLAT: FP64 chunks that look uniform take the copy that leaves out what is zero
+// on uniform planes; its checks cost a mixed plane 5 %, so the others take the
+// plain one.  FP32 runs the one copy with those checks, for the same reason as
+// above (with both, 256x256x512 takes 1.23 ms a step, against 1.06).
 template <typename S, int L, int TY, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool SPLIT, bool PHASE, bool FAST,
-          int HQ>
+          int HQ, bool FLAT>
 __device__ __forceinline__ bool march_any(const DomainDesc& d, const KC<S>& c, const KC<typename Lanes<S, L>::V>& cv,
-                                          const CUtensorMap* tm, const S* c_in, S* phi_out, S* dpp, S* c_out,
-                                          const S* T_old, S* T_new, int zchunk, int bx, int by, int bz,
+                                          const CUtensorMap* tm, const S* phi_in, const S* c_in, S* phi_out, S* dpp,
+                                          S* c_out, const S* T_old, S* T_new, int zchunk, int bx, int by, int bz,
                                           unsigned char* smem, uint32_t& par)
 {
     const int x0 = bx * 32, y0 = by * TY;
     constexpr bool copies = sizeof(S) == 8;
-    if (copies && x0 >= 3 && x0 + 32 + 3 <= d.nx && y0 >= 3 && y0 + TY + 3 <= d.ny)
-        return march_tile<S, L, TY, HEAT, DPPW, SOL, SMOOTH, SPLIT, PHASE, FAST, HQ, true>(
+    const bool inside = copies && x0 >= 3 && x0 + 32 + 3 <= d.nx && y0 >= 3 && y0 + TY + 3 <= d.ny;
+    if constexpr (FLAT && copies) {
+        if (inside && looks_flat<S>(d, phi_in, x0, y0, bz * zchunk, min(bz * zchunk + zchunk, d.nz)))
+            return march_tile<S, L, TY, HEAT, DPPW, SOL, SMOOTH, SPLIT, PHASE, FAST, HQ, true, true>(
+                d, c, cv, tm, c_in, phi_out, dpp, c_out, T_old, T_new, zchunk, bx, by, bz, smem, par);
+    }
+    if (inside)
+        return march_tile<S, L, TY, HEAT, DPPW, SOL, SMOOTH, SPLIT, PHASE, FAST, HQ, false, true>(
             d, c, cv, tm, c_in, phi_out, dpp, c_out, T_old, T_new, zchunk, bx, by, bz, smem, par);
-    return march_tile<S, L, TY, HEAT, DPPW, SOL, SMOOTH, SPLIT, PHASE, FAST, HQ, false>(
+    return march_tile<S, L, TY, HEAT, DPPW, SOL, SMOOTH, SPLIT, PHASE, FAST, HQ, FLAT && !copies, false>(
         d, c, cv, tm, c_in, phi_out, dpp, c_out, T_old, T_new, zchunk, bx, by, bz, smem, par);
 }
 
@@ -615,10 +719,12 @@ struct MarchOcc {
 };
 
 // single domain: one CTA per tile; the phase field comes through `tm`
-template <typename S, int L, int TY, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool PHASE, bool FAST, int HQ>
+template <typename S, int L, int TY, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool PHASE, bool FAST, int HQ,
+          bool FLAT>
 __global__ void __launch_bounds__(32 * TY / L, (MarchOcc<S, L, PHASE, FAST, HEAT && SOL>::v))
     k_march(const __grid_constant__ CUtensorMap tm, DomainDesc d, const KC<S> c,
-            const KC<typename Lanes<S, L>::V> cv, const S* __restrict__ c_in, S* __restrict__ phi_out,
+            const KC<typename Lanes<S, L>::V> cv, const S* __restrict__ phi_in, const S* __restrict__ c_in,
+            S* __restrict__ phi_out,
             S* __restrict__ dpp, S* __restrict__ c_out, const S* __restrict__ T_old, S* __restrict__ T_new,
             int zchunk, int* __restrict__ err)
 {
@@ -628,8 +734,8 @@ __global__ void __launch_bounds__(32 * TY / L, (MarchOcc<S, L, PHASE, FAST, HEAT
     march_init_barriers<MarchLayout<S, TY, SOL, PHASE, FAST>>(smem);
     pdl_wait();
     uint32_t par = 0;
-    if (!march_any<S, L, TY, HEAT, DPPW, SOL, SMOOTH, sizeof(S) == 8, PHASE, FAST, HQ>(
-            d, c, cv, &tm, c_in, phi_out, dpp, c_out, T_old, T_new, zchunk, blockIdx.x, blockIdx.y, blockIdx.z, smem,
+    if (!march_any<S, L, TY, HEAT, DPPW, SOL, SMOOTH, sizeof(S) == 8, PHASE, FAST, HQ, FLAT>(
+            d, c, cv, &tm, phi_in, c_in, phi_out, dpp, c_out, T_old, T_new, zchunk, blockIdx.x, blockIdx.y, blockIdx.z, smem,
             par)) {
         if (threadIdx.x == 0 && threadIdx.y == 0) atomicExch(err, kErrTmaTimeout);
     }
@@ -697,17 +803,17 @@ __global__ void __launch_bounds__(32 * TY / L, (MarchOcc<S, L, true, true, ONE_S
         if (PASS == 0) {
             const CUtensorMap* tm = tmaps + 2 * it.dom + q;
             if (ONE_SWEEP)
-                ok = march_any<S, L, TY, true, true, true, SMOOTH, false, true, true, 2>(
-                    D.d, skc, kv, tm, (const S*)D.c[qc], (S*)D.phi[1 - q], (S*)D.dpp, (S*)D.c[1 - qc],
+                ok = march_any<S, L, TY, true, true, true, SMOOTH, false, true, true, 2, false>(
+                    D.d, skc, kv, tm, nullptr, (const S*)D.c[qc], (S*)D.phi[1 - q], (S*)D.dpp, (S*)D.c[1 - qc],
                     (const S*)D.T[qt], (S*)D.T[1 - qt], zchunk, it.bx, it.by, it.bz, smem, par);
             else
-                ok = march_any<S, L, TY, true, false, false, SMOOTH, false, true, true, 2>(
-                    D.d, skc, kv, tm, (const S*)D.c[qc], (S*)D.phi[1 - q], (S*)D.dpp, nullptr, (const S*)D.T[qt],
+                ok = march_any<S, L, TY, true, false, false, SMOOTH, false, true, true, 2, false>(
+                    D.d, skc, kv, tm, nullptr, (const S*)D.c[qc], (S*)D.phi[1 - q], (S*)D.dpp, nullptr, (const S*)D.T[qt],
                     (S*)D.T[1 - qt], zchunk, it.bx, it.by, it.bz, smem, par);
         } else {
             const CUtensorMap* tm = tmaps + 2 * it.dom + (1 - q);
-            ok = march_any<S, L, TY, false, true, true, false, false, true, true, 2>(
-                D.d, skc, kv, tm, (const S*)D.c[qc], (S*)D.phi[q], (S*)D.dpp, (S*)D.c[1 - qc], nullptr, nullptr,
+            ok = march_any<S, L, TY, false, true, true, false, false, true, true, 2, false>(
+                D.d, skc, kv, tm, nullptr, (const S*)D.c[qc], (S*)D.phi[q], (S*)D.dpp, (S*)D.c[1 - qc], nullptr, nullptr,
                 zchunk, it.bx, it.by, it.bz, smem, par);
         }
         if (!ok) {
@@ -745,13 +851,15 @@ KC<typename Lanes<S, L>::V> kc_lanes(const KC<S>& k)
     }
 }
 
-template <typename S, int L, int TY, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool PHASE, bool FAST, int HQ>
-cudaError_t launch_march_t(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s, const void* c_in,
+template <typename S, int L, int TY, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool PHASE, bool FAST, int HQ,
+          bool FLAT = false>
+cudaError_t launch_march_t(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s, const void* phi_in,
+                           const void* c_in,
                            void* phi_out, void* dpp, void* c_out, const void* T_old, void* T_new, int zchunk,
                            int* err, cudaStream_t st)
 {
     using LY = MarchLayout<S, TY, SOL, PHASE, FAST>;
-    auto kern = k_march<S, L, TY, HEAT, DPPW, SOL, SMOOTH, PHASE, FAST, HQ>;
+    auto kern = k_march<S, L, TY, HEAT, DPPW, SOL, SMOOTH, PHASE, FAST, HQ, FLAT>;
     static bool configured = false;   // one attribute call per instantiation
     if (!configured) {
         cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::ALLOC);
@@ -763,40 +871,55 @@ cudaError_t launch_march_t(const CUtensorMap& tm, const DomainDesc& d, const Ste
     kc.load(d, s);
     const auto kv = kc_lanes<S, L>(kc);
     dim3 grid((d.nx + 31) / 32, (d.ny + TY - 1) / TY, (d.nz + zchunk - 1) / zchunk);
-    return launch_pdl(kern, grid, dim3(32, TY / L), LY::ALLOC, st, tm, d, kc, kv, (const S*)c_in, (S*)phi_out,
+    return launch_pdl(kern, grid, dim3(32, TY / L), LY::ALLOC, st, tm, d, kc, kv, (const S*)phi_in, (const S*)c_in, (S*)phi_out,
                       (S*)dpp, (S*)c_out, (const S*)T_old, (S*)T_new, zchunk, err);
 }
 
 // the passes of a step (32 x 8 tiles).  lanes: cells per thread (1 or 2); the
 // smooth noise runs one cell per thread.  h(phi) is known at compile time.
+//
+// flat: with what serves uniform planes.  How much of a domain is uniform grows
+// with its depth around the interface (in a run under way the FP64 phase is
+// exactly 1 some 37 cells inside the crystal, the FP32 phase also exactly 0 some
+// 105 cells into the melt; a young run's melt is exactly 0 altogether), and a
+// chunk learns of its first planes' uniformity four planes late.  So it serves
+// domains of kFlatDepth planes and chunks of kFlatChunk and more, of steps with
+// two sweeps (with more, a middle sweep may need the noise of a cell the first
+// one left alone).  Measured, without / with: crystal a third grown, 340x340x700
+// FP64 4.23 / 4.14 ms a step, 256x256x512 FP32 1.089 / 1.063 ms, but 192x192x384
+// FP32 0.567 / 0.588 ms and 340x340x200 FP64 1.29 / 1.32 ms; seeded start,
+// 512x512x1024 FP64 12.6 / 8.9 ms, 1024^3 FP32 27.6 / 19.6 ms.
 template <typename S>
 cudaError_t launch_march_first(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s, const Fields& f,
-                               bool with_solute, int lanes, int zchunk, int* err, cudaStream_t st)
+                               bool with_solute, int lanes, bool flat, int zchunk, int* err, cudaStream_t st)
 {
-#define PF3D_MF(L, SO, SM, HQ)                                                                                  \
-    launch_march_t<S, L, 8, true, SO, SO, SM, true, true, HQ>(tm, d, s, f.c_old, f.phi_mid, f.dpp,              \
-                                                              SO ? f.c_new : nullptr, f.T_old, f.T_new, zchunk, \
-                                                              err, st)
-#define PF3D_MQ(L, SO) (d.hq ? PF3D_MF(L, SO, false, 1) : PF3D_MF(L, SO, false, 0))
-    if (d.rt == 2) {
-        if (with_solute) return d.hq ? PF3D_MF(1, true, true, 1) : PF3D_MF(1, true, true, 0);
-        return d.hq ? PF3D_MF(1, false, true, 1) : PF3D_MF(1, false, true, 0);
-    }
-    if (with_solute) return lanes == 2 ? PF3D_MQ(2, true) : PF3D_MQ(1, true);
-    return lanes == 2 ? PF3D_MQ(2, false) : PF3D_MQ(1, false);
+#define PF3D_MF(L, SO, SM, HQ, FL)                                                                              \
+    launch_march_t<S, L, 8, true, SO, SO, SM, true, true, HQ, FL>(tm, d, s, f.phi_old, f.c_old, f.phi_mid, f.dpp, \
+                                                                  SO ? f.c_new : nullptr, f.T_old, f.T_new,     \
+                                                                  zchunk, err, st)
+#define PF3D_MQ(L, SO, SM, FL) (d.hq ? PF3D_MF(L, SO, SM, 1, FL) : PF3D_MF(L, SO, SM, 0, FL))
+    constexpr int L0 = sizeof(S) == 4 ? 2 : 1;   // the default lanes, which the flat copies have
+    if (d.rt == 2) return with_solute ? PF3D_MQ(1, true, true, false) : PF3D_MQ(1, false, true, false);
+    if (with_solute) return lanes == 2 ? PF3D_MQ(2, true, false, false) : PF3D_MQ(1, true, false, false);
+    if (flat && lanes == L0) return PF3D_MQ(L0, false, false, true);
+    return lanes == 2 ? PF3D_MQ(2, false, false, false) : PF3D_MQ(1, false, false, false);
 #undef PF3D_MQ
 #undef PF3D_MF
 }
 
 template <typename S>
 cudaError_t launch_march_last(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s, const Fields& f,
-                              int lanes, int zchunk, int* err, cudaStream_t st)
+                              int lanes, bool flat, int zchunk, int* err, cudaStream_t st)
 {
-#define PF3D_ML(L, HQ)                                                                                          \
-    launch_march_t<S, L, 8, false, true, true, false, true, true, HQ>(tm, d, s, f.c_old, f.phi_new, f.dpp,     \
-                                                                      f.c_new, nullptr, nullptr, zchunk, err, st)
-    if (lanes == 2) return d.hq ? PF3D_ML(2, 1) : PF3D_ML(2, 0);
-    return d.hq ? PF3D_ML(1, 1) : PF3D_ML(1, 0);
+#define PF3D_ML(L, HQ, FL)                                                                                      \
+    launch_march_t<S, L, 8, false, true, true, false, true, true, HQ, FL>(tm, d, s, f.phi_mid, f.c_old, f.phi_new, f.dpp, \
+                                                                          f.c_new, nullptr, nullptr, zchunk,   \
+                                                                          err, st)
+#define PF3D_MQ(L, FL) (d.hq ? PF3D_ML(L, 1, FL) : PF3D_ML(L, 0, FL))
+    constexpr int L0 = sizeof(S) == 4 ? 2 : 1;
+    if (flat && lanes == L0) return PF3D_MQ(L0, true);
+    return lanes == 2 ? PF3D_MQ(2, false) : PF3D_MQ(1, false);
+#undef PF3D_MQ
 #undef PF3D_ML
 }
 
@@ -815,7 +938,7 @@ cudaError_t launch_march_sweep(const CUtensorMap& tm, const DomainDesc& d, const
     constexpr bool FAST = sizeof(S) == 4;
     const bool smooth = d.rt == 2;
 #define PF3D_MS(DW, SM)                                                                                          \
-    launch_march_t<S, 1, 8, false, DW, false, SM, true, FAST, 2>(tm, d, s, c_in, phi_out, dpp, nullptr, nullptr, \
+    launch_march_t<S, 1, 8, false, DW, false, SM, true, FAST, 2>(tm, d, s, nullptr, c_in, phi_out, dpp, nullptr, nullptr, \
                                                                  nullptr, zchunk, err, st)
     if (dpp) return smooth ? PF3D_MS(true, true) : PF3D_MS(true, false);
     return smooth ? PF3D_MS(false, true) : PF3D_MS(false, false);
@@ -827,7 +950,7 @@ cudaError_t launch_march_solute(const CUtensorMap& tm, const DomainDesc& d, cons
                                 void* c_out, int zchunk, int* err, cudaStream_t st)
 {
     return launch_march_t<S, 1, 8, false, false, true, false, false, sizeof(S) == 4, 2>(
-        tm, d, s, c_in, nullptr, nullptr, c_out, nullptr, nullptr, zchunk, err, st);
+        tm, d, s, nullptr, c_in, nullptr, nullptr, c_out, nullptr, nullptr, zchunk, err, st);
 }
 
 // The persistent grid is the SM count times the CTAs of this kernel that are

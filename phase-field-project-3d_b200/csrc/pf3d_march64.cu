@@ -4,6 +4,6 @@
 #include "pf3d_march.cuh"
 
 namespace pf3d {
-template cudaError_t launch_march_first<double>(const CUtensorMap&, const DomainDesc&, const StepArgs&, const Fields&, bool, int, int, int*, cudaStream_t);
-template cudaError_t launch_march_last<double>(const CUtensorMap&, const DomainDesc&, const StepArgs&, const Fields&, int, int, int*, cudaStream_t);
+template cudaError_t launch_march_first<double>(const CUtensorMap&, const DomainDesc&, const StepArgs&, const Fields&, bool, int, bool, int, int*, cudaStream_t);
+template cudaError_t launch_march_last<double>(const CUtensorMap&, const DomainDesc&, const StepArgs&, const Fields&, int, bool, int, int*, cudaStream_t);
 }  // namespace pf3d
