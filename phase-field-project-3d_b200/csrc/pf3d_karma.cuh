@@ -158,6 +158,7 @@ struct KarmaWindow {
                 p[r * KT::W + c] = p[rr * KT::W + cc];
             }
         }
+        fence_proxy_async_smem();   // before the barrier that lets a later load overwrite these cells
     }
 };
 
@@ -288,10 +289,7 @@ __global__ void __launch_bounds__(32 * TY, (KarmaOcc<T>::v))
             }
             return;
         }
-        if (lead && z + 3 <= ze) {
-            fence_proxy_async_smem();
-            w.issue(q + 4);
-        }
+        if (lead && z + 3 <= ze) w.issue(q + 4);   // into a slot only read since its last barrier
     }
 }
 
@@ -421,10 +419,7 @@ __global__ void __launch_bounds__(32 * TY, (KarmaOcc<T>::v))
             }
             return;
         }
-        if (lead && z + 3 <= ze) {
-            fence_proxy_async_smem();
-            w.issue(s + 4);
-        }
+        if (lead && z + 3 <= ze) w.issue(s + 4);   // into a slot only read since its last barrier
     }
 }
 
