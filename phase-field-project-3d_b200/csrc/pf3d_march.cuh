@@ -179,7 +179,8 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
     constexpr int NRING = (L == 1) ? 2 * NW + 2 * TY : NW + TY;  // ring items (pairs when L = 2)
     constexpr int NT = 32 * TY / L;
     static_assert(TY % L == 0, "tile height must be a multiple of the lanes");
-    static_assert(2 * NRING <= NT, "the node and solute ring threads are disjoint");
+    constexpr int NOUT = FLAT ? (2 * TX + 2 * TY) / L : 0;       // second halo's items (FLAT)
+    static_assert(2 * NRING + NOUT <= NT, "the threads of the two rings and of the second halo are disjoint");
 
     const uint32_t sb = smem_u32(smem);
     const uint32_t bar0 = sb + LY::BAR_OFF;
@@ -201,13 +202,27 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
     const uint32_t own_phi = (uint32_t)((ty + 2) * PR + (tx + XOFF) * ES);   // lane 0, in a phase slot
     const uint32_t own_node = (uint32_t)((ty + 1) * NR + (tx + 1) * ES);     // lane 0, in a node array
     const bool ring = tid < NRING;                      // ring nodes
+    const bool outer = FLAT && tid >= NRING && tid < NRING + NOUT;   // second halo's phase values
     const bool ring_s = SOL && tid >= NT - NRING;       // ring solute points
     uint32_t col[L], rcol[L];      // element offsets in the plane: own cells, ring points
-    uint32_t rphi[L], rnode[L];    // bytes from the thread's own position (lane 0) to its ring items
+    uint32_t rphi[L], rnode[L];    // bytes from the thread's own position (lane 0) to its ring (or second halo) items
     bool own[L], xyin[L], rin[L], rdom[L];
     {
         int r = ring ? tid : (ring_s ? tid - (NT - NRING) : 0), rx[L], ry[L];
-        if (L == 1) {
+        if (outer) {   // what the ring's nodes read beyond the ring, without corners
+            r = tid - NRING;
+            if (L == 1) {
+                const bool lo = r < TX + TY;
+                if (!lo) r -= TX + TY;
+                rx[0] = r < TX ? 1 + r : (lo ? -1 : NW);
+                ry[0] = r < TX ? (lo ? -1 : NH) : 1 + (r - TX);
+            } else {
+                rx[0] = r < TX ? 1 + r : -1;
+                ry[0] = r < TX ? -1 : 1 + (r - TX);
+                rx[L - 1] = r < TX ? 1 + r : NW;
+                ry[L - 1] = r < TX ? NH : 1 + (r - TX);
+            }
+        } else if (L == 1) {
             if (r < NW) { rx[0] = r; ry[0] = 0; }
             else if ((r -= NW) < NW) { rx[0] = r; ry[0] = NH - 1; }
             else if ((r -= NW) < TY) { rx[0] = 0; ry[0] = 1 + r; }
@@ -226,7 +241,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
             const int x = x0 + tx, y = y0 + ty + l * TR, gx = x0 - 1 + rx[l], gy = y0 - 1 + ry[l];
             own[l] = INT || (x < nx && y < ny);
             xyin[l] = INT || (x >= 1 && x <= nx - 2 && y >= 1 && y <= ny - 2);
-            rdom[l] = ring && (INT || (gx >= 0 && gx < nx && gy >= 0 && gy < ny));    // its phase value counts
+            rdom[l] = (ring || outer) && (INT || (gx >= 0 && gx < nx && gy >= 0 && gy < ny));    // its phase value counts
             rin[l] = ring_s && (INT || (gx >= 0 && gx < nx && gy >= 0 && gy < ny));   // its concentration is read
             col[l] = (uint32_t)x + (uint32_t)y * (uint32_t)px;
             rcol[l] = (uint32_t)gx + (uint32_t)gy * (uint32_t)px;
@@ -404,9 +419,10 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
     uint32_t am = phi_at((zb + 5) % 6), a0 = phi_at(zb % 6), ap = phi_at((zb + 1) % 6);   // planes z-1, z, z+1
     int sq = (zb + 2) % 6;       // phase slot of plane z+2
     long long zoff = zo0;
-    // what planes z-1, z and z+1 hold all over the tile and its ring (inside the
-    // domain): 1 exactly 0, 2 exactly 1, 0 anything else or not known yet
-    int un = 0, u0 = 0, u1 = 0;
+    // what planes z-2 .. z+1 hold all over the tile and its 2-cell halo (inside
+    // the domain), two bits a plane, z+1 in the lowest: 1 exactly 0, 2 exactly 1,
+    // 0 anything else or not known yet
+    int uh = 0;
 
     // One plane of the march.  IN: every z-dependent condition of the plane
     // is known true (z in [3, N-4], the planes it reads and the load it
@@ -432,13 +448,13 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
         // concentrations of plane z keep the driving force's logarithm finite
         // (0 < c < Ke); and whether the warp's nodes of plane z+1 are flat
         bool mixed = false, own_flat = false, ring_flat = false;
-        int u2 = u1;
+        int u2 = uh & 3;
         if constexpr (FLAT) {
             if (IN || z + 2 <= zlast) {
                 S v;
                 lds(sb + (uint32_t)(sq * LY::PHI_BYTES + 2 * PR + XOFF * ES), v);   // the tile's first cell
                 u2 = is_bits0(v) ? 1 : is_bits1(v) ? 2 : 0;
-                bool od = false, rd = false;   // own cells, ring items that differ from it
+                bool od = false, rd = false;   // own cells, ring and second halo items that differ from it
 #pragma unroll
                 for (int l = 0; l < L; ++l) {
                     S a, b;
@@ -448,7 +464,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
                     rd = rd || (rdom[l] && b != v);
                 }
                 mixed = u2 == 0 || od || rd;
-                if (u0 != 0 && u0 == u1 && u1 == u2) {   // planes z and z+1 hold it too (CTA-uniform)
+                if (u2 != 0 && (uh & 15) == 5 * u2) {   // planes z and z+1 hold it too (CTA-uniform)
                     own_flat = !__any_sync(0xffffffffu, od);
                     ring_flat = !__any_sync(0xffffffffu, rd);
                 }
@@ -481,16 +497,17 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
         // only, by threads that are behind the barrier)
         if (lead && (IN || z + 4 <= zlast)) issue(z + 4, sq + 2 >= 6 ? sq - 4 : sq + 2);
 
-        // F: the cells of plane z.  Where planes z-1 .. z+2 hold nothing but 0 or
+        // F: the cells of plane z.  Where all that their sweep reads -- planes
+        // z-2 .. z+2 of the tile and its 2-cell halo -- holds nothing but 0 or
         // nothing but 1, every difference, g', h' and the noise's
         // phi^2 (1-phi)^2 are zero and the sweep changes nothing: the cells
         // keep their value and DPP is zero, the bits the arithmetic gives as
         // long as its logarithm is finite.  (The noise is not drawn either:
-        // the second sweep multiplies it by the same zero.)
-        const bool flat = FLAT && un != 0 && un == u0 && u0 == u1 && u1 == u2;
-        un = u0;
-        u0 = u1;
-        u1 = u2;
+        // the second sweep multiplies it by the same zero.)  All that is read
+        // counts, not only what the zeros multiply: a node beside a NaN makes
+        // NaN of a zero difference.
+        if constexpr (FLAT) uh = ((uh << 2) | u2) & 0x3ff;
+        const bool flat = FLAT && u2 != 0 && uh == 0x155 * u2;
         const bool zi = IN || zin(z);                     // T interior / phase source / solute interior
         const bool zph = IN || (z >= 2 && z <= nz - 3);   // phase interior
         const V PP = ldv(a0, 0, false);
