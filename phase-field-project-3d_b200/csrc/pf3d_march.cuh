@@ -446,7 +446,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
         if (IN || z + 2 <= zlast) bad |= !wait_plane(sq);
         // whether plane z+2 holds one of the two values all over, and the
         // concentrations of plane z keep the driving force's logarithm finite
-        // (0 < c < Ke); and whether the warp's nodes of plane z+1 are flat
+        // (KC::cflat); and whether the warp's nodes of plane z+1 are flat
         bool mixed = false, own_flat = false, ring_flat = false;
         int u2 = uh & 3;
         if constexpr (FLAT) {
@@ -470,7 +470,7 @@ __device__ __forceinline__ bool march_tile(const DomainDesc& d, const KC<S>& c, 
                 }
             }
 #pragma unroll
-            for (int l = 0; l < L; ++l) mixed = mixed || (own[l] && !(co[l] > (S)0 && co[l] < c.Ke));
+            for (int l = 0; l < L; ++l) mixed = mixed || (own[l] && !(co[l] > (S)0 && co[l] < c.cflat));
         }
         // B, C: nodes and solute points of plane z+1
         if (PHASE && (IN || zin(z + 1))) node_plane(np, a0, ap, aq, own_flat, ring_flat);
