@@ -46,6 +46,10 @@ KarmaK<T> karma_constants(const pf_karma_params& p)
     c.Ahalf2 = (T)(0.5 * (1.0 - p.k));
     c.D = (T)(kA2 * p.lambda);
     c.at = (T)kAt;
+    // zero differences times every factor of dphi's expression, over as^2 (0/0
+    // for eps4 = 1/3), and the noise's zero amplitude
+    c.z0 = (T)0 * (c.idx + c.q + c.h + c.om3 * c.om3 + c.lambda) / (c.om3 * c.om3);
+    if (c.Fnoise != (T)0) c.z0 = c.z0 + c.Fnoise * (T)0 / c.sqdt;
     return c;
 }
 

@@ -61,6 +61,7 @@ struct KarmaK {
     T Ahalf2;     // 0.5*(1-k)
     T D;          // a2*lambda
     T at;         // 1/(2 sqrt 2)
+    T z0;         // dphi without the term in U where phi is +1 or -1 all around: 0, or NaN where a parameter makes it so
 };
 
 template <typename T>
@@ -240,7 +241,7 @@ __global__ void __launch_bounds__(32 * TY, (KarmaOcc<T>::v))
         const int ut = k_uniform3<T, W>(w.plane(0, q + 2), o, oe, o0, own);
         if (up != 0 && ub == up && ut == up) {
             // every gradient and 1 - phi^2 are zero: dphi = 0 (0 times U keeps a non-finite U visible)
-            if (own) dphi[id] = (T)0 * uc + (T)0;
+            if (own) dphi[id] = c.z0 * uc + c.z0;
         } else if (own) {
             const T* const B = w.plane(0, q) + o;
             const T pp = P[0];
