@@ -58,7 +58,7 @@ def test_no_diffusion_in_the_solid_steps(gpu, sweeps, fused):
 
 
 @pytest.mark.parametrize("small", [1e-160, 1e-250, 1e-300])
-@pytest.mark.parametrize("fused,kernel", [(0, 1)])
+@pytest.mark.parametrize("fused,kernel", [(0, 1), (1, 1), (1, 0)])
 def test_vanishing_concentration(gpu, fused, kernel, small):
     """A block of cells with next to no solute, inside the melt and across tiles:
     the reference gives finite values there, and so does every form."""
