@@ -187,9 +187,14 @@ int pf_create(const pf_grid* g, const pf_params* p, int precision, pf_ctx** out)
     ctx->d_track = (unsigned long long*)(ctx->d_out + 8);
     ctx->d_track_out = (double*)(ctx->d_track + round_up((size_t)g->nz + 1, 4));
     ctx->d_status = (int*)(ctx->d_track_out + 4);
-    if ((e = cudaMemset(ctx->base, 0, total)) != cudaSuccess ||
-        (e = cudaMallocHost(&ctx->h_out, 8 * sizeof(double))) != cudaSuccess ||
-        (e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking)) != cudaSuccess) {
+    // cleared on the context's own stream and waited for: it does not order
+    // itself after the default stream, nor does one the caller sets later
+    if ((e = cudaMallocHost(&ctx->h_out, 8 * sizeof(double))) != cudaSuccess ||
+        (e = cudaStreamCreateWithFlags(&ctx->own_stream, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = cudaMemsetAsync(ctx->base, 0, total, ctx->own_stream)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(ctx->own_stream)) != cudaSuccess) {
+        if (ctx->own_stream) cudaStreamDestroy(ctx->own_stream);
+        cudaFreeHost(ctx->h_out);
         cudaFree(ctx->base);
         delete ctx;
         return set_global_err(PF_E_CUDA, std::string("context set-up: ") + cudaGetErrorString(e));

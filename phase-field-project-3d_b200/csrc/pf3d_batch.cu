@@ -402,10 +402,16 @@ int pf_batch_create(int precision, long long budget_bytes, int max_domains, pf_b
         }
         cudaGetLastError();
     }
-    cudaMemset(b->d_steps, 0, step_bytes);
-    cudaMemset(b->d_nitems, 0, 2 * sizeof(int));
-    cudaMemset(b->d_status, 0, sizeof(int));
-    cudaMemset(b->d_part, 0, (592 * kDiagRow + 8) * sizeof(double));   // the diagnostics' block counter among it
+    // cleared on the batch's own stream and waited for (pf_create)
+    if ((e = cudaMemsetAsync(b->d_steps, 0, step_bytes, b->stream)) != cudaSuccess ||
+        (e = cudaMemsetAsync(b->d_nitems, 0, 2 * sizeof(int), b->stream)) != cudaSuccess ||
+        (e = cudaMemsetAsync(b->d_status, 0, sizeof(int), b->stream)) != cudaSuccess ||
+        // the diagnostics' block counter is in d_part
+        (e = cudaMemsetAsync(b->d_part, 0, (592 * kDiagRow + 8) * sizeof(double), b->stream)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(b->stream)) != cudaSuccess) {
+        pf_batch_destroy(b);
+        return set_last_error_global(PF_E_CUDA, std::string("pf_batch_create: ") + cudaGetErrorString(e));
+    }
     if (!tmap_encoder()) b->march = 0;   // no tensor-map encoder in this driver: the cp.async passes
     set_grid(b);
     *out = b;

@@ -176,9 +176,13 @@ int pf_karma_create(const pf_karma_params* p, int precision, pf_karma** out)
         delete k;
         return kerr(PF_E_CUDA, "tensor map encoding failed");
     }
-    if ((e = cudaMemset(k->base, 0, 5 * k->field_bytes + 256)) != cudaSuccess ||
-        (e = cudaMallocHost(&k->h_tip, 3 * sizeof(int))) != cudaSuccess ||
-        (e = cudaStreamCreateWithFlags(&k->own_stream, cudaStreamNonBlocking)) != cudaSuccess) {
+    // cleared on the object's own stream and waited for (pf_create)
+    if ((e = cudaMallocHost(&k->h_tip, 3 * sizeof(int))) != cudaSuccess ||
+        (e = cudaStreamCreateWithFlags(&k->own_stream, cudaStreamNonBlocking)) != cudaSuccess ||
+        (e = cudaMemsetAsync(k->base, 0, 5 * k->field_bytes + 256, k->own_stream)) != cudaSuccess ||
+        (e = cudaStreamSynchronize(k->own_stream)) != cudaSuccess) {
+        if (k->own_stream) cudaStreamDestroy(k->own_stream);
+        cudaFreeHost(k->h_tip);
         cudaFree(k->base);
         delete k;
         return kerr(PF_E_CUDA, std::string("set-up: ") + cudaGetErrorString(e));
