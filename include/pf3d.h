@@ -144,10 +144,11 @@ int pf_set_stream(pf_ctx* ctx, void* stream);
 #define PF_OPT_FUSED 1     /* 1 (default): pf_step uses the fused kernels;
                               0: it calls the per-subroutine kernels        */
 #define PF_OPT_TILE_Y 2    /* fused tile height: 4, 8 (default) or 16       */
-#define PF_OPT_ZCHUNK 3    /* z planes per fused CTA (0 = whole column); until
-                              it is set (default 64) the TMA passes take the
-                              chunk that fills the GPU with the domain's
-                              tiles.  Same results.                         */
+#define PF_OPT_ZCHUNK 3    /* z planes per fused CTA (0 = whole column).  At 64,
+                              the default, the TMA passes take the chunk that
+                              fills the GPU with the domain's tiles.  The
+                              passes that run one subroutine alone (middle
+                              sweeps among them) always do.  Same results.  */
 #define PF_OPT_KTIMING 4   /* 1: time every fused launch with CUDA events   */
 #define PF_OPT_PAIRED 5    /* two cells per thread on 32 x 8 fused tiles
                               (same results): 1 (default) in FP32, where it
@@ -320,8 +321,8 @@ int pf_batch_step_async(pf_batch* b, int n_steps);
 int pf_batch_wait(pf_batch* b);
 /* device milliseconds of the last pf_batch_step call (all its graphs)      */
 double pf_batch_last_ms(const pf_batch* b);
-/* tile height and z-chunk; until set (or autotuned) tiles are 32 x 8 and the
-   TMA passes take the chunk that suits the batch's membership               */
+/* tile height and z-chunk, 8 and 64 by default; with a chunk of 64 the TMA
+   passes take the one that suits the batch's membership.  Same results.     */
 int pf_batch_set_tile(pf_batch* b, int tile_y, int zchunk);
 /* 32 x 8 tiles: 1 runs two cells per thread (same results), 0 one; until set,
    two in FP32 batches on the TMA passes, else one.  The

@@ -73,7 +73,7 @@ struct pf_ctx {
     cudaStream_t own_stream;
     cudaStream_t stream;
     int fused, tile_y, zchunk, ktiming, paired;
-    int zchunk_set;          // PF_OPT_ZCHUNK was set; until then the march passes' chunk is fill_zchunk's
+    int zchunk_set;          // PF_OPT_ZCHUNK is not its default; at the default the march passes' chunk is fill_zchunk's
     int zfill[3];            // ... cached by the CTAs an SM holds (index: kMarchOcc)
     int n_sm;
     int kernel;              // PF_OPT_KERNEL: 1 TMA-staged march passes, 0 the cp.async passes
@@ -158,7 +158,7 @@ int pf_create(const pf_grid* g, const pf_params* p, int precision, pf_ctx** out)
     fill_desc(*g, *p, ctx->dv, px, ctx->dd);
     ctx->fused = 1;
     ctx->tile_y = 8;
-    ctx->zchunk = 64;
+    ctx->zchunk = kZChunkDefault;
     ctx->ktiming = 0;
     ctx->paired = 1;
     cudaGetDevice(&ctx->device);
@@ -300,7 +300,7 @@ int pf_set_option(pf_ctx* ctx, int opt, int value)
     case PF_OPT_ZCHUNK:
         if (value < 0) return ctx_err(ctx, PF_E_ARG, "zchunk must be >= 0");
         ctx->zchunk = value;
-        ctx->zchunk_set = 1;
+        ctx->zchunk_set = value != kZChunkDefault;
         return PF_OK;
     case PF_OPT_KTIMING: ctx->ktiming = value ? 1 : 0; return PF_OK;
     case PF_OPT_PAIRED:

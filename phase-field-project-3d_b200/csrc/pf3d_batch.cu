@@ -82,8 +82,7 @@ struct pf_batch {
     int track_cap = 0;                 // planes it holds
     double* h_out = nullptr;
     double* d_sites = nullptr;         // bump sites for device initialisation
-    int tile_y = 8, zchunk = 64, n_sm = 0;   // persistent grids: n_sm x resident CTAs
-    bool zauto = true;                 // the chunk follows the membership (batch_zchunk) until a tile is set
+    int tile_y = 8, zchunk = kZChunkDefault, n_sm = 0;   // persistent grids: n_sm x resident CTAs
     int zc = 64;                       // chunk of the current work list
     int pair = -1;                     // 32 x 8 tiles with two cells per thread; -1: FP32 yes, FP64 no
     int march = 1;                     // TMA-staged march passes (32 x 8 tiles); 0: the cp.async passes
@@ -157,7 +156,8 @@ static bool use_march(const pf_batch* b) { return b->march && b->tile_y == 8; }
 
 static int rebuild_items(pf_batch* b)
 {
-    b->zc = b->zauto && use_march(b) ? batch_zchunk(b) : b->zchunk;
+    // the default chunk is the rule's on the TMA passes
+    b->zc = b->zchunk == kZChunkDefault && use_march(b) ? batch_zchunk(b) : b->zchunk;
     std::vector<BatchItem> items;
     // largest domains first: their items are the longest-running
     std::vector<int> order;
@@ -688,8 +688,7 @@ int pf_batch_set_tile(pf_batch* b, int tile_y, int zchunk)
 {
     if (!b || (tile_y != 4 && tile_y != 8 && tile_y != 16) || zchunk < 1)
         return berr(b, PF_E_ARG, "pf_batch_set_tile: tile_y in {4, 8, 16}, zchunk >= 1");
-    if (b->zauto || tile_y != b->tile_y || zchunk != b->zchunk) {
-        b->zauto = false;
+    if (tile_y != b->tile_y || zchunk != b->zchunk) {
         b->tile_y = tile_y;
         b->zchunk = zchunk;
         b->items_dirty = true;

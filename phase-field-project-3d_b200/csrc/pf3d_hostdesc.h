@@ -87,6 +87,9 @@ inline int validate(const pf_grid* g, const pf_params* p, int precision, std::st
 // 217 -> 22 us a step, 64x64x128 FP64 291 -> 58 us, 150x111x190 FP32
 // 343 -> 160 us, 256x256x512 FP32 1.22 -> 1.15 ms, 340x340x700 FP64 unchanged.
 constexpr int kZChunkMax = 128;
+// the value a chunk option reports and starts with, and the one that leaves the
+// chunk to the library: so an option that is saved and restored is as it was
+constexpr int kZChunkDefault = 64;
 inline int fill_zchunk(long long tiles, int nz, int n_sm, int occ, double pro, double grow)
 {
     int best_zc = nz < kZChunkMax ? nz : kZChunkMax;
