@@ -334,12 +334,14 @@ int pf_batch_set_paired(pf_batch* b, int paired);
    TMA-staged passes on 32 x 8 tiles, 0 the element-wise cp.async passes;
    nslot as PF_OPT_NSLOT                                                  */
 int pf_batch_set_kernel(pf_batch* b, int kernel, int nslot);
-/* Autotuner: times every tile shape x z-chunk (16, 32, 64, 128) x one or
+/* Autotuner: times every tile shape x z-chunk (16, 32, 64, 128; 64 is the
+   batch's own choice on the TMA passes) x one or
    two cells per thread -- tile heights 4, 8 and 16 for the cp.async passes,
    32 x 8 for the TMA passes -- on real steps (the results do not depend on
    these choices; each candidate advances the batch by 1 +
    steps_per_candidate steps), keeps the fastest and caches it per shape
-   class (precision, median column size and depth)                         */
+   class (precision, median column size and depth).  Where no slot has a step
+   left to time, nothing changes and nothing is cached                     */
 int pf_batch_autotune(pf_batch* b, int steps_per_candidate, int* tile_y, int* zchunk, double* ms_per_step);
 /* pf_diagnosticos of one slot's state (the watchdog as there)             */
 int pf_batch_diagnosticos(pf_batch* b, int slot, double out[5]);

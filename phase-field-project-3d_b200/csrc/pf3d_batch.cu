@@ -797,7 +797,7 @@ int pf_batch_autotune(pf_batch* b, int steps_per_candidate, int* tile_y, int* zc
         auto it = g_tune_cache.find(key);
         if (it != g_tune_cache.end()) {
             int rc = pf_batch_set_tile(b, std::get<0>(it->second), std::get<1>(it->second));
-            b->pair = std::get<2>(it->second);
+            if (!rc) rc = pf_batch_set_paired(b, std::get<2>(it->second));
             if (tile_y) *tile_y = std::get<0>(it->second);
             if (zchunk) *zchunk = std::get<1>(it->second);
             if (ms_per_step) *ms_per_step = -1.0;
@@ -805,19 +805,31 @@ int pf_batch_autotune(pf_batch* b, int steps_per_candidate, int* tile_y, int* zc
         }
     }
     // every candidate runs real steps (results do not depend on the tile
-    // shape), one untimed step first
+    // shape), one untimed step first.  The chunk of 64 planes stands for the
+    // membership's own (batch_zchunk) on the TMA passes, so the choice in use
+    // by default is among the candidates.  The batch is left as it was unless
+    // a candidate has been timed.
     double best = 1e300;
-    int bty = b->tile_y, bzc = b->zchunk, bpair = want_pair(b);
+    const int ty0 = b->tile_y, zc0 = b->zchunk, pair0 = b->pair;
+    int bty = ty0, bzc = zc0, bpair = pair0;
+    auto restore = [&] {
+        pf_batch_set_tile(b, ty0, zc0);
+        b->pair = pair0;
+        b->items_dirty = true;
+    };
     const bool march = b->march != 0;
     for (int ty : {4, 8, 16})
         for (int zc : {16, 32, 64, 128})
             for (int pr = 0; pr <= ((ty == 8 && (march || !b64(b))) ? 1 : 0); ++pr) {
                 if (march && ty != 8) break;   // the march passes run 32 x 8 tiles
                 int rc = pf_batch_set_tile(b, ty, zc);
-                b->pair = pr;
+                if (!rc) rc = pf_batch_set_paired(b, pr);
                 if (!rc) rc = pf_batch_step(b, 1);
                 if (!rc) rc = pf_batch_step(b, steps_per_candidate);
-                if (rc) return rc;
+                if (rc) {
+                    restore();
+                    return rc;
+                }
                 if (b->last_steps == 0) break;
                 const double ms = b->last_ms / (double)b->last_steps;
                 if (ms < best) {
@@ -827,11 +839,14 @@ int pf_batch_autotune(pf_batch* b, int steps_per_candidate, int* tile_y, int* zc
                     bpair = pr;
                 }
             }
-    int rc = pf_batch_set_tile(b, bty, bzc);
-    b->pair = bpair;
-    {
+    int rc = PF_OK;
+    if (best < 1e300) {
+        rc = pf_batch_set_tile(b, bty, bzc);
+        if (!rc) rc = pf_batch_set_paired(b, bpair);
         std::lock_guard<std::mutex> lk(g_tune_mu);
         g_tune_cache[key] = std::make_tuple(bty, bzc, bpair);
+    } else {
+        restore();   // every slot had reached its target
     }
     if (tile_y) *tile_y = bty;
     if (zchunk) *zchunk = bzc;

@@ -3,7 +3,8 @@ the option and the batch report and start with, and it means the library's
 choice: saving and restoring the option, or setting a batch's default tile,
 must leave the passes as fast as one that was never touched (a fixed 64-plane
 chunk is some ten times slower on the domain below), and an explicit chunk
-changes no bit."""
+changes no bit.  The autotuner must not end slower than the choice it starts
+from, nor keep what it did not time."""
 import numpy as np
 import pytest
 
@@ -99,3 +100,25 @@ def test_batch_tile_restored(gpu):
         b.step(1)
         b.set_tile(8, 64)
         assert batch_us(b) < SLACK * plain
+
+
+def test_autotune_is_not_slower_and_keeps_only_what_it_timed(gpu):
+    g, p, st = setup()
+    with pf3d.Batch(pf3d.PF_FP64) as b:
+        s = b.add(g, p)
+        b.load_state(s, st)
+        b.set_target(s, 1)
+        b.step(1)                       # the slot has reached its target: nothing to time
+        plain_it = b.state(s).it
+        b.autotune(1)
+        assert b.state(s).it == plain_it
+        b.set_target(s, 0)
+        untimed = batch_us(b)
+    with pf3d.Batch(pf3d.PF_FP64) as b:
+        s = b.add(g, p)
+        b.load_state(s, st)
+        plain = batch_us(b)
+        assert untimed < SLACK * plain
+        _, _, ms = b.autotune(20)
+        assert ms > 0                   # timed here, not taken from the call that timed nothing
+        assert batch_us(b) < 1.5 * plain
