@@ -84,6 +84,42 @@ cudaError_t run_thread(const Job& j, int t, int nt)
     return e;
 }
 
+// without the chunks: the driver's copy, FP32 through one conversion
+cudaError_t direct(const Job& j)
+{
+    const size_t row = (size_t)j.nx * j.es;
+    std::vector<float> f;
+    void* buf = j.host;
+    if (j.es == 4) {
+        try {
+            f.resize((size_t)j.nx * j.n_rows);
+        } catch (...) {
+            return cudaErrorMemoryAllocation;
+        }
+        buf = f.data();
+        if (!j.to_host)
+            for (size_t q = 0; q < f.size(); ++q) f[q] = (float)j.host[q];
+    }
+    cudaError_t e = j.to_host ? cudaMemcpy2DAsync(buf, row, j.dev, (size_t)j.px * j.es, row, (size_t)j.n_rows,
+                                                  cudaMemcpyDeviceToHost, j.stream)
+                              : cudaMemcpy2DAsync(j.dev, (size_t)j.px * j.es, buf, row, row, (size_t)j.n_rows,
+                                                  cudaMemcpyHostToDevice, j.stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(j.stream);
+    if (e == cudaSuccess && j.to_host)
+        for (size_t q = 0; q < f.size(); ++q) j.host[q] = (double)f[q];
+    return e;
+}
+
+// chunk t is there, or could be allocated
+bool have_chunk(int t)
+{
+    if (!g_buf[t] && cudaHostAlloc(&g_buf[t], kChunk, cudaHostAllocPortable) != cudaSuccess) {
+        g_buf[t] = nullptr;
+        cudaGetLastError();
+    }
+    return g_buf[t] != nullptr;
+}
+
 cudaError_t transfer(Job j)
 {
     cudaError_t e = cudaStreamSynchronize(j.stream);
@@ -91,43 +127,24 @@ cudaError_t transfer(Job j)
     const size_t row = (size_t)j.nx * j.es;
     const size_t bytes = row * (size_t)j.n_rows;
     const bool small = (size_t)j.nx * j.n_rows * 8 < (j.es == 8 ? kSmall64 : kSmall32);
-    if (j.es == 8 && (small || row > kChunk)) {
-        e = j.to_host ? cudaMemcpy2DAsync(j.host, row, j.dev, (size_t)j.px * 8, row, (size_t)j.n_rows,
-                                          cudaMemcpyDeviceToHost, j.stream)
-                      : cudaMemcpy2DAsync(j.dev, (size_t)j.px * 8, j.host, row, row, (size_t)j.n_rows,
-                                          cudaMemcpyHostToDevice, j.stream);
-        return e == cudaSuccess ? cudaStreamSynchronize(j.stream) : e;
-    }
-    if (small || row > kChunk) {   // FP32 outside the chunks' range: one conversion through a vector
-        std::vector<float> f;
-        try {
-            f.resize((size_t)j.nx * j.n_rows);
-        } catch (...) {
-            return cudaErrorMemoryAllocation;
-        }
-        if (!j.to_host)
-            for (size_t q = 0; q < f.size(); ++q) f[q] = (float)j.host[q];
-        e = j.to_host ? cudaMemcpy2DAsync(f.data(), row, j.dev, (size_t)j.px * 4, row, (size_t)j.n_rows,
-                                          cudaMemcpyDeviceToHost, j.stream)
-                      : cudaMemcpy2DAsync(j.dev, (size_t)j.px * 4, f.data(), row, row, (size_t)j.n_rows,
-                                          cudaMemcpyHostToDevice, j.stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(j.stream);
-        if (e == cudaSuccess && j.to_host)
-            for (size_t q = 0; q < f.size(); ++q) j.host[q] = (double)f[q];
-        return e;
-    }
+    if (small || row > kChunk) return direct(j);
     e = cudaGetDevice(&j.device);
     if (e != cudaSuccess) return e;
     // equal chunks, at least one a thread where the field is large enough
     const int hw = (int)std::max(1u, std::thread::hardware_concurrency() / 2);
-    const int nt = (int)std::min<size_t>(std::min(kXferThreads, hw), (bytes + (1u << 20) - 1) >> 20);
+    int nt = (int)std::min<size_t>(std::min(kXferThreads, hw), (bytes + (1u << 20) - 1) >> 20);
     long long n_chunks = (long long)((bytes + kChunk - 1) / kChunk);
     n_chunks = (n_chunks + nt - 1) / nt * nt;
     j.rows_per = std::max<long long>(1, (j.n_rows + n_chunks - 1) / n_chunks);
     j.rows_per = std::min<long long>(j.rows_per, (long long)(kChunk / row));
-    std::lock_guard<std::mutex> lk(g_mu);
-    for (int t = 0; t < nt; ++t)
-        if (!g_buf[t] && (e = cudaHostAlloc(&g_buf[t], kChunk, cudaHostAllocPortable)) != cudaSuccess) return e;
+    std::unique_lock<std::mutex> lk(g_mu);
+    int have = 0;
+    while (have < nt && have_chunk(have)) ++have;
+    if (have == 0) {   // no pinned memory to be had
+        lk.unlock();
+        return direct(j);
+    }
+    nt = have;
     cudaError_t rc[kXferThreads] = {};
     std::thread thr[kXferThreads];
     int started = 1;
