@@ -128,8 +128,11 @@ cudaError_t transfer(Job j)
     const size_t bytes = row * (size_t)j.n_rows;
     const bool small = (size_t)j.nx * j.n_rows * 8 < (j.es == 8 ? kSmall64 : kSmall32);
     if (small || row > kChunk) return direct(j);
-    e = cudaGetDevice(&j.device);
+    // the field's device, which need not be the calling thread's
+    cudaPointerAttributes at;
+    e = cudaPointerGetAttributes(&at, j.dev);
     if (e != cudaSuccess) return e;
+    j.device = at.device;
     // equal chunks, at least one a thread where the field is large enough
     const int hw = (int)std::max(1u, std::thread::hardware_concurrency() / 2);
     int nt = (int)std::min<size_t>(std::min(kXferThreads, hw), (bytes + (1u << 20) - 1) >> 20);
@@ -155,8 +158,11 @@ cudaError_t transfer(Job j)
         }
     } catch (...) {   // no more threads: this one takes the shares that are left
     }
+    int own = j.device;
+    cudaGetDevice(&own);
     for (int t = started; t < nt; ++t) rc[t] = run_thread(j, t, nt);
     rc[0] = run_thread(j, 0, nt);
+    if (own != j.device) cudaSetDevice(own);
     for (int t = 1; t < started; ++t) thr[t].join();
     for (int t = 0; t < nt; ++t)
         if (rc[t] != cudaSuccess) e = rc[t];

@@ -162,3 +162,13 @@ def test_delivers_without_pinned_chunks(harness, es, nx, rows, allowed):
     made all the same, and no error is left behind."""
     r = result(harness("copy", es, nx, rows, allowed, 1))
     assert (r["up"], r["down"], r["bad"], r["left"], r["live"]) == (0, 0, 0, 0, 0), r
+
+
+@pytest.mark.parametrize("es", [8, 4])
+@pytest.mark.parametrize("nx,rows", SIZES)
+def test_field_of_another_device(harness, es, nx, rows):
+    """The calling thread's current device is not the field's (a thread that
+    only reads fields back): the transfer runs on the field's device, and the
+    thread keeps its own."""
+    r = result(harness("copy", es, nx, rows, 100, 0))
+    assert (r["up"], r["down"], r["bad"], r["left"], r["live"], r["device"]) == (0, 0, 0, 0, 0, 0), r
