@@ -110,13 +110,18 @@ cudaError_t direct(const Job& j)
     return e;
 }
 
-// chunk t is there, or could be allocated
+// chunk t is there, or could be allocated (in the relaxed capture mode: while
+// another thread captures a graph, an allocation is refused in the default one)
 bool have_chunk(int t)
 {
-    if (!g_buf[t] && cudaHostAlloc(&g_buf[t], kChunk, cudaHostAllocPortable) != cudaSuccess) {
+    if (g_buf[t]) return true;
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    cudaThreadExchangeStreamCaptureMode(&mode);
+    if (cudaHostAlloc(&g_buf[t], kChunk, cudaHostAllocPortable) != cudaSuccess) {
         g_buf[t] = nullptr;
         cudaGetLastError();
     }
+    cudaThreadExchangeStreamCaptureMode(&mode);
     return g_buf[t] != nullptr;
 }
 

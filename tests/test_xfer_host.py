@@ -172,3 +172,11 @@ def test_field_of_another_device(harness, es, nx, rows):
     thread keeps its own."""
     r = result(harness("copy", es, nx, rows, 100, 0))
     assert (r["up"], r["down"], r["bad"], r["left"], r["live"], r["device"]) == (0, 0, 0, 0, 0, 0), r
+
+
+def test_allocates_beside_a_capture(harness):
+    """Another thread may be capturing a graph, during which an allocation in the
+    default capture mode fails (and can end the capture): the chunks are
+    allocated in the relaxed mode."""
+    r = result(harness("copy", 8, 200, 9000, 100, 1))
+    assert r["allocations"] > 0 and r["unsafe"] == 0, r
