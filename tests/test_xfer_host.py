@@ -53,7 +53,7 @@ static thread_local cudaError_t t_err = cudaSuccess;
 static thread_local cudaStreamCaptureMode t_mode = cudaStreamCaptureModeGlobal;
 static std::atomic<int> n_alloc{0}, live{0}, unsafe{0};
 static int allocs_allowed = 1 << 30;
-static const char *dev_lo, *dev_hi, *pin_lo, *pin_hi;
+static const char *dev_lo, *dev_hi;
 static const int kDevice = 1;                       // where the field and its stream live
 static cudaError_t ret(cudaError_t e) { if (e != cudaSuccess) t_err = e; return e; }
 
@@ -87,33 +87,25 @@ cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void* p)
 {
     const char* c = (const char*)p;
     if (c >= dev_lo && c < dev_hi) *a = {cudaMemoryTypeDevice, kDevice};
-    else if (c >= pin_lo && c < pin_hi) *a = {cudaMemoryTypeHost, 0};
     else *a = {cudaMemoryTypeUnregistered, -2};
     return cudaSuccess;
 }
 cudaError_t cudaGetLastError() { cudaError_t e = t_err; t_err = cudaSuccess; return e; }
 cudaError_t cudaThreadExchangeStreamCaptureMode(cudaStreamCaptureMode* m) { std::swap(*m, t_mode); return cudaSuccess; }
 
-// argv: what, element size, nx, rows, allocations allowed, the caller's device
+// argv: element size, nx, rows, allocations allowed, the caller's device
 int main(int argc, char** argv)
 {
-    const std::string what = argv[1];
-    const int es = std::atoi(argv[2]), nx = std::atoi(argv[3]);
-    const long long rows = std::atoll(argv[4]), px = (nx + 31) / 32 * 32;
-    allocs_allowed = std::atoi(argv[5]);
-    cudaSetDevice(std::atoi(argv[6]));
+    const int es = std::atoi(argv[1]), nx = std::atoi(argv[2]);
+    const long long rows = std::atoll(argv[3]), px = (nx + 31) / 32 * 32;
+    allocs_allowed = std::atoi(argv[4]);
+    cudaSetDevice(std::atoi(argv[5]));
     FakeStream st{kDevice};
     std::vector<char> dev((size_t)px * rows * es, 77);
     std::vector<double> a((size_t)nx * rows), b(a.size(), -1.0);
     dev_lo = dev.data();
     dev_hi = dev_lo + dev.size();
-    pin_lo = (const char*)a.data();
-    pin_hi = pin_lo + 1;
     for (size_t i = 0; i < a.size(); ++i) a[i] = (double)(i * 2654435761u % 1000003) / 997.0 - 300.0;
-    if (what == "reach") {   // which arrays the copy engines reach without staging
-        std::printf("%d %d %d\n", pf3d::xfer_pinned(a.data()), pf3d::xfer_pinned(dev.data()), pf3d::xfer_pinned(b.data()));
-        return 0;
-    }
     pf3d::xfer_ref();
     const cudaError_t up = pf3d::xfer_to_device(dev.data(), es, nx, px, rows, a.data(), &st);
     const cudaError_t down = pf3d::xfer_to_host(dev.data(), es, nx, px, rows, b.data(), &st);
@@ -134,7 +126,7 @@ int main(int argc, char** argv)
 def harness(tmp_path_factory):
     d = tmp_path_factory.mktemp("xfer")
     (d / "cuda_runtime.h").write_text(RUNTIME)
-    (d / "main.cpp").write_text("#include <string>\n#include <utility>\n" + HARNESS)
+    (d / "main.cpp").write_text("#include <utility>\n" + HARNESS)
     exe = str(d / "xfer")
     subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I", str(d), "-I", CSRC, str(d / "main.cpp"), "-x", "c++",
                     os.path.join(CSRC, "pf3d_xfer.cu"), "-o", exe], check=True)
@@ -160,7 +152,7 @@ SIZES = [(4, 1), (33, 7000), (200, 9000), (131, 20011), (140000, 9)]
 def test_delivers_without_pinned_chunks(harness, es, nx, rows, allowed):
     """The staging chunks cannot be allocated, or only some of them: the copy is
     made all the same, and no error is left behind."""
-    r = result(harness("copy", es, nx, rows, allowed, 1))
+    r = result(harness(es, nx, rows, allowed, 1))
     assert (r["up"], r["down"], r["bad"], r["left"], r["live"]) == (0, 0, 0, 0, 0), r
 
 
@@ -170,7 +162,7 @@ def test_field_of_another_device(harness, es, nx, rows):
     """The calling thread's current device is not the field's (a thread that
     only reads fields back): the transfer runs on the field's device, and the
     thread keeps its own."""
-    r = result(harness("copy", es, nx, rows, 100, 0))
+    r = result(harness(es, nx, rows, 100, 0))
     assert (r["up"], r["down"], r["bad"], r["left"], r["live"], r["device"]) == (0, 0, 0, 0, 0, 0), r
 
 
@@ -178,5 +170,5 @@ def test_allocates_beside_a_capture(harness):
     """Another thread may be capturing a graph, during which an allocation in the
     default capture mode fails (and can end the capture): the chunks are
     allocated in the relaxed mode."""
-    r = result(harness("copy", 8, 200, 9000, 100, 1))
+    r = result(harness(8, 200, 9000, 100, 1))
     assert r["allocations"] > 0 and r["unsafe"] == 0, r
