@@ -33,6 +33,7 @@
 #pragma once
 #include <type_traits>
 #include "pf3d_launch.h"
+#include "pf3d_once.h"
 #include "pf3d_pair.cuh"
 #include "pf3d_tma.cuh"
 
@@ -877,12 +878,10 @@ cudaError_t launch_march_t(const CUtensorMap& tm, const DomainDesc& d, const Ste
 {
     using LY = MarchLayout<S, TY, SOL, PHASE, FAST>;
     auto kern = k_march<S, L, TY, HEAT, DPPW, SOL, SMOOTH, PHASE, FAST, HQ, FLAT>;
-    static bool configured = false;   // one attribute call per instantiation
-    if (!configured) {
-        cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::ALLOC);
-        if (e != cudaSuccess) return e;
-        configured = true;
-    }
+    static DeviceOnce once;   // one attribute call per instantiation and device
+    const cudaError_t e = once(
+        [&] { return cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, LY::ALLOC); });
+    if (e != cudaSuccess) return e;
     if (zchunk <= 0) zchunk = d.nz;
     KC<S> kc;
     kc.load(d, s);
