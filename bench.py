@@ -60,17 +60,18 @@ def step_hbm_frac_of(gbs: float, peak: float) -> float:
     return gbs / peak
 
 
-def ncu_figures(kernel: str, precision: int) -> dict:
-    """Per-cell figures of a fused pass from the committed ncu summary
-    (profiles/ncu_passes.txt: `<pass> fp<NN> key=value ...`): DRAM bytes,
-    executed thread instructions and FP64 flops per cell, issue-active and
-    FP64-pipe fractions of the captured launch."""
+def ncu_figures(workload: str, kernel: str) -> dict:
+    """Per-cell figures of a fused pass on this very workload from the
+    committed ncu summary (profiles/ncu_passes.txt: `<workload> <pass>
+    key=value ...`): DRAM bytes, executed thread instructions and FP64-pipe
+    instructions per cell.  Empty for a workload that has not been captured:
+    they depend on how much of a domain is uniform."""
     path = os.path.join(ROOT, "profiles", "ncu_passes.txt")
     out = {}
     try:
         for line in open(path):
             t = line.split()
-            if len(t) >= 3 and not t[0].startswith("#") and t[0] == kernel and t[1] == f"fp{precision}":
+            if len(t) >= 3 and not t[0].startswith("#") and t[:2] == [workload, kernel]:
                 for kv in t[2:]:
                     k, v = kv.split("=")
                     out[k] = float(v)
@@ -399,37 +400,33 @@ def main():
     alg_bytes = PASS_BYTES_PER_CELL[kname][prec] * cells
     avg_s = ms_k / max(1, n_k) / 1e3
     achieved = alg_bytes / avg_s / 1e9
-    fig = ncu_figures(kname, prec)
+    fig = ncu_figures(w.name, kname)
     tr = fig.get("dram_bytes_per_cell")
     step_gbs = value / world * STEP_BYTES_PER_CELL[prec]
-    # the other two ceilings of the dominant pass, from this run's kernel time
-    # and the per-cell counts of its ncu capture: the FP64 pipe (nominal peak
+    # the ceilings of the dominant pass, from this run's kernel time and the
+    # per-cell counts of its ncu capture on the same workload: HBM, the FP64 pipe (nominal peak
     # 148 SMs x 64 FP64 FMA a clock x 2 flops at the sampled SM clock) and
     # instruction issue (148 SMs x 4 schedulers x 1 warp instruction a clock)
     clk_hz = (clk["sm_mhz"] if clk and clk.get("sm_mhz") else 1965.0) * 1e6
     n_sm = torch.cuda.get_device_properties(local).multi_processor_count
-    ceilings = {"hbm": (tr * cells / avg_s / 1e9) / peak if tr else achieved / peak}
+    ceilings = {"hbm": (tr * cells / avg_s / 1e9) / peak} if tr else {}
     fp64 = None
     if prec == 64 and "fp64_inst_per_cell" in fig:
-        # FP64 pipe: lane-operations (DFMA, DMUL, DADD) per second against
-        # 64 a clock per SM; flops count an FMA as two
+        # FP64 pipe: lane-operations per second against 64 a clock per SM
         peak_ops = n_sm * 64 * clk_hz
         ops = fig["fp64_inst_per_cell"] * cells / avg_s
-        other = ncu_figures("fused_first" if kname == "fused_last" else "fused_last", prec)
+        other = ncu_figures(w.name, "fused_first" if kname == "fused_last" else "fused_last")
         step_ops = (fig["fp64_inst_per_cell"] + other.get("fp64_inst_per_cell", 0.0)) * cells * args.steps / (ms / 1e3)
-        step_flops = fig.get("fp64_flops_per_cell", 0.0) + other.get("fp64_flops_per_cell", 0.0)
-        fp64 = {"achieved_tflops": fig.get("fp64_flops_per_cell", 0.0) * cells / avg_s / 1e12,
-                "peak_tflops": 2 * peak_ops / 1e12, "pipe_frac": ops / peak_ops,
-                "inst_per_cell": fig["fp64_inst_per_cell"], "flops_per_cell": fig.get("fp64_flops_per_cell"),
+        fp64 = {"peak_tflops": 2 * peak_ops / 1e12, "pipe_frac": ops / peak_ops,
+                "inst_per_cell": fig["fp64_inst_per_cell"],
                 "step": {"inst_per_cell": fig["fp64_inst_per_cell"] + other.get("fp64_inst_per_cell", 0.0),
-                         "flops_per_cell": step_flops, "pipe_frac": step_ops / peak_ops,
-                         "achieved_tflops": step_flops * cells * args.steps / (ms / 1e3) / 1e12},
+                         "pipe_frac": step_ops / peak_ops},
                 "peak_source": f"nominal: {n_sm} SMs x 64 FP64 lane-operations a clock at the sampled "
                                f"{clk_hz / 1e6:.0f} MHz"}
         ceilings["fp64_pipe"] = ops / peak_ops
     if "inst_per_cell" in fig:
         ceilings["issue"] = fig["inst_per_cell"] / 32 * cells / avg_s / (n_sm * 4 * clk_hz)
-    limiter = max(ceilings, key=ceilings.get)
+    limiter = max(ceilings, key=ceilings.get) if ceilings else None
     roofline = {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                 "traffic": (tr * cells if tr is not None else None), "kernel": kname,
                 "kernel_ms": avg_s * 1e3, "peak_source": f"{peak_kind} hbm_gbs",

@@ -17,7 +17,9 @@
 //    one barrier a plane (MarchLayout).
 //  * Uniform arithmetic, fan-out stores.  Every cell of every tile -- also
 //    the tiles on the domain boundary -- goes through the same arithmetic
-//    (two cells per thread as lane pairs when L = 2, packed f32x2 in FP32).
+//    (two cells per thread as lane pairs when L = 2, packed f32x2 in FP32),
+//    in copies of the body that differ in their checks only; in deep domains
+//    the cells of a uniform plane keep their value instead (FLAT).
 //    The boundary decoration of the reference (plane copies after the sweep,
 //    equacao_campo_fase.f90:151-167, concentracao_soluto.f90:116-124) is a
 //    per-cell store fan-out: a cell writes its value to every cell whose
@@ -143,9 +145,9 @@ __device__ __forceinline__ void march_init_barriers(unsigned char* smem)
 // second store (FP64).
 // PHASE = false leaves the phase sweep out (the solute subroutine alone);
 // FAST = false is the reference form of the per-subroutine entry points (FP64,
-// one lane).  FLAT: planes on which the tile holds nothing but 0 or nothing but
-// 1 (melt beyond the interface's tail, the crystal's interior) leave out what
-// is exactly zero there (two-sweep steps, below).
+// one lane).  FLAT: planes on which the tile and its 2-cell halo hold nothing but
+// 0 or nothing but 1 (melt beyond the interface's tail, the crystal's interior)
+// leave out what is exactly zero there (two-sweep steps, below).
 //
 // The arithmetic is a third to a half of what a plane executes: the rest is
 // addresses, conditions and moves, and every thread repeats it in every
@@ -703,7 +705,7 @@ __device__ __forceinline__ bool looks_flat(const DomainDesc& d, const S* phi, in
 // FLAT: FP64 chunks that look uniform take the copy that leaves out what is zero
 // on uniform planes; its checks cost a mixed plane 5 %, so the others take the
 // plain one.  FP32 runs the one copy with those checks, for the same reason as
-// above (with both, 256x256x512 takes 1.23 ms a step, against 1.06).
+// above (with both, 256x256x512 took 1.23 ms a step, against 1.06).
 template <typename S, int L, int TY, bool HEAT, bool DPPW, bool SOL, bool SMOOTH, bool SPLIT, bool PHASE, bool FAST,
           int HQ, bool FLAT>
 __device__ __forceinline__ bool march_any(const DomainDesc& d, const KC<S>& c, const KC<typename Lanes<S, L>::V>& cv,
@@ -901,10 +903,14 @@ cudaError_t launch_march_t(const CUtensorMap& tm, const DomainDesc& d, const Ste
 // chunk learns of its first planes' uniformity four planes late.  So it serves
 // domains of kFlatDepth planes and chunks of kFlatChunk and more, of steps with
 // two sweeps (with more, a middle sweep may need the noise of a cell the first
-// one left alone).  Measured, without / with: crystal a third grown, 340x340x700
-// FP64 4.23 / 4.14 ms a step, 256x256x512 FP32 1.089 / 1.063 ms, but 192x192x384
-// FP32 0.567 / 0.588 ms and 340x340x200 FP64 1.29 / 1.32 ms; seeded start,
-// 512x512x1024 FP64 12.6 / 8.9 ms, 1024^3 FP32 27.6 / 19.6 ms.
+// one left alone).  The depth stands in for the state, which the host does not
+// know; the line lies where a grown crystal begins to gain.  Microseconds a step,
+// without / with.  Crystal a third grown: FP64 340x340 x 200 1294 / 1326, x 330
+// 2069 / 2103, x 448 2847 / 2895, x 700 4236 / 4150; FP32 192x192 x 256 380 / 387,
+// x 384 572 / 581, x 448 663 / 667, 256x256 x 512 1096 / 1040, x 700 1533 / 1447.
+// Seeded start: FP64 192x192 x 200 470 / 481, x 384 880 / 902, 256x256x512
+// 1864 / 1629, 512x512x1024 12648 / 8959; FP32 192x192 x 200 302 / 267, x 384
+// 571 / 476, 256x256x512 1096 / 870, 1024^3 27723 / 18911.
 template <typename S>
 cudaError_t launch_march_first(const CUtensorMap& tm, const DomainDesc& d, const StepArgs& s, const Fields& f,
                                bool with_solute, int lanes, bool flat, int zchunk, int* err, cudaStream_t st)
